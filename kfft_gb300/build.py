@@ -24,7 +24,13 @@ LIB_DIR = os.path.join(HERE, "lib")
 OBJ_DIR = os.path.join(HERE, "_build")
 SOURCES = ["pass_smem.cu", "pass_reg.cu", "persistent.cu", "tables.cu", "plan.cu", "api.cu",
            "uneven.cu", "noalloc.cu", "helpers.cu", "mlp.cu"]
-HEADERS = ["engine.cuh", "fft_device.cuh", "plan_host.h"]
+# Double build only: its fixed-point pass kernels, in parts that compile in
+# parallel, and the FP64 tile they and the queue kernel call.  These share
+# device code across objects (-rdc), the FP64 tile within 64 registers.
+FX_SOURCES = [("fp64_tile.cu", "fp64_tile", ["-maxrregcount=64"])]
+FX_SOURCES += [("pass_fx.cu", f"pass_fx{p}", [f"-DKFFT_FX_PART={p}"]) for p in range(4)]
+RDC = {"persistent.cu", "fp64_tile.cu", "pass_fx.cu"}
+HEADERS = ["engine.cuh", "fft_device.cuh", "fx_math.cuh", "fx_spec.cuh", "fx_tile.cuh", "plan_host.h"]
 ARCH = ["-gencode", "arch=compute_103a,code=sm_103a"]
 VARIANTS = {"libkfft_gb300.so": [], "libkfft_gb300_f.so": ["-DKFFT_HALF_SCALAR"]}
 
@@ -55,7 +61,7 @@ def _compile(src: str, obj: str, defines: list[str]) -> None:
 def build(force: bool = False, verbose: bool = False) -> dict[str, str]:
     os.makedirs(LIB_DIR, exist_ok=True)
     os.makedirs(OBJ_DIR, exist_ok=True)
-    deps = [os.path.join(CSRC, s) for s in SOURCES + HEADERS]
+    deps = [os.path.join(CSRC, s) for s in SOURCES + HEADERS + [f[0] for f in FX_SOURCES]]
     deps += [os.path.join(ROOT, "include", h) for h in ("kfft.h", "kfft_gb300.h")]
     out = {}
     jobs = []
@@ -66,10 +72,12 @@ def build(force: bool = False, verbose: bool = False) -> dict[str, str]:
             continue
         tag = lib.replace(".so", "")
         objs = []
-        for s in SOURCES:
-            obj = os.path.join(OBJ_DIR, f"{tag}_{s.replace('.cu', '.o')}")
+        units = [(s, s[:-3], []) for s in SOURCES] + ([] if defines else FX_SOURCES)
+        for s, name, more in units:
+            obj = os.path.join(OBJ_DIR, f"{tag}_{name}.o")
             objs.append(obj)
-            jobs.append((os.path.join(CSRC, s), obj, defines))
+            rdc = ["-rdc=true"] if s in RDC and not defines else []
+            jobs.append((os.path.join(CSRC, s), obj, defines + more + rdc))
         jobs.append(("LINK", target, objs))
     compile_jobs = [j for j in jobs if j[0] != "LINK"]
     with cf.ThreadPoolExecutor(max_workers=min(16, os.cpu_count() or 4)) as ex:

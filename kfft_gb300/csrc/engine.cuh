@@ -52,6 +52,18 @@ struct FastDiv {
     void init(uint32_t div);
 };
 
+// A number of modulus at most 1 in two signed 32-bit limbs a part, value *
+// 2^62 = h * 2^32 + l: the tables of the double build's fixed-point tiles.
+struct alignas(16) FxTw {
+    int32_t rh, rl, ih, il;
+};
+// elements a thread of a fixed-point tile holds at most
+constexpr uint32_t kFxElems = 16;
+// rows of lane words a fixed-point tile has at least (one a stage)
+constexpr uint32_t kFxRows = 4;
+// threads of a full power-of-two fixed-point tile (8 points each)
+constexpr uint32_t kFxSpecThreads = 512;
+
 enum : uint8_t { MODE_LANE = 0, MODE_ELEM = 1 };
 enum : uint8_t { ORDER_J = 0, ORDER_B = 1 };
 
@@ -113,9 +125,33 @@ struct PassDesc {
     uint64_t aux_in_bs, aux_out_bs;
     uint32_t aux_out_es;
     real_t scale;
+#if !defined(KFFT_HALF_SCALAR)
+    // fixed-point tile (fx_tile.cuh): forward tables in two-limb form
+    uint8_t fx;             // the tile runs in fixed point
+    uint8_t inplace;        // three or more stages of one butterfly a thread: one exchange buffer
+    uint32_t fx_words;      // byte offset of the lane words in shared memory
+    const FxTw* fx_inner;   // tw_inner's forward twiddles
+    const FxTw* fx_lo;      // tw_lo's and tw_hi's
+    const FxTw* fx_hi;
+    const FxTw* fx_pro;     // pro_tab (chirp)
+    const FxTw* fx_epi;     // epi_tab (chirp, or a spectrum scaled by 2^-fx_epi_e)
+    int32_t fx_epi_e;
+    int32_t fx_scale_h, fx_scale_l;  // scale = 2^fx_scale_e, times these limbs / 2^62 unless zero
+    int32_t fx_scale_e;
+#endif
 };
 
 // ---- device tables -----------------------------------------------------
+#if !defined(KFFT_HALF_SCALAR)
+// Two-limb tables of the fixed-point tiles, exact to a few 2^-62: forward
+// twiddles exp(-2 pi i (i * mult mod n) / n), the chirp of gen_chirp, and a
+// spectrum divided by the power of two *exp (written on the device; its
+// largest part then lies in [1/4, 1/2)).
+void gen_fx_twiddles(FxTw* t, uint32_t count, uint64_t mult, uint32_t n, cudaStream_t st);
+void gen_fx_chirp(FxTw* c, uint32_t count, uint32_t n, int sign, cudaStream_t st);
+void gen_fx_spectrum(FxTw* t, const vec2_t* spectrum, uint32_t count, int32_t* exp,
+                     cudaStream_t st);
+#endif
 // Fills t[i] = exp(sign * 2 pi i * (i * mult mod n) / n) in FP64 for i < count.
 void gen_twiddles(vec2_t* t, uint32_t count, uint64_t mult, uint32_t n, int sign,
                   cudaStream_t st);
@@ -187,6 +223,9 @@ struct PassSpec {
     uint32_t R, Ns;
     std::vector<uint8_t> radices;
     const vec2_t* tw_inner;
+#if !defined(KFFT_HALF_SCALAR)
+    const FxTw* fx_inner;
+#endif
 };
 
 struct DeviceArena;  // device memory owned by a plan tree
@@ -235,6 +274,13 @@ struct FftPlan {
     const uint32_t* gperm = nullptr;  // Rader: g^j mod p
     const uint32_t* iperm = nullptr;  // Rader: g^-j mod p
     uint32_t generator = 0;
+#if !defined(KFFT_HALF_SCALAR)
+    const FxTw* fx_lo = nullptr;       // two-limb forms of the tables above
+    const FxTw* fx_hi = nullptr;
+    const FxTw* fx_chirp = nullptr;
+    const FxTw* fx_spectrum = nullptr;
+    int32_t fx_spectrum_e = 0;
+#endif
     ~FftPlan();
 };
 

@@ -479,12 +479,15 @@ __device__ __forceinline__ void store_elem(const PassDesc& d, uint32_t b, uint32
             break;
         case EPI_RADER_FWD:
             // spectrum of the gathered sequence times the kernel spectrum; bin 0
-            // is sum_{n>=1} x_n, so X_0 = x_0 + v is saved with x_0 per sequence
-            d.out[b * d.out_bs + uint64_t(k) * d.out_es] = cmul(v, __ldg(&d.epi_tab[k]));
+            // is sum_{n>=1} x_n, so X_0 = x_0 + v is saved per sequence, and x_0
+            // added to bin 0 of the product adds x_0 to every output of the
+            // (unnormalised) inverse
             if (k == 0) {
                 const vec2_t x0 = __ldcg(&d.aux_in[b * d.aux_in_bs]);
-                d.aux_out[2 * uint64_t(b)] = x0;
-                d.aux_out[2 * uint64_t(b) + 1] = cadd(x0, v);
+                d.aux_out[b] = cadd(x0, v);
+                d.out[b * d.out_bs] = cadd(cmul(v, __ldg(&d.epi_tab[0])), x0);
+            } else {
+                d.out[b * d.out_bs + uint64_t(k) * d.out_es] = cmul(v, __ldg(&d.epi_tab[k]));
             }
             break;
         case EPI_MUL_OUT: {
@@ -493,13 +496,12 @@ __device__ __forceinline__ void store_elem(const PassDesc& d, uint32_t b, uint32
             break;
         }
         case EPI_RADER_INV: {
-            // X[g^-k] = x_0 + c_k, and X_0 from the saved pair; never reads the input,
+            // X[g^-k] = v (x_0 is in it), and the saved X_0; never reads the input,
             // so the transform may run in place
-            const vec2_t x0 = __ldcg(&d.aux_in[2 * uint64_t(b)]);
             const uint32_t idx = __ldg(&d.epi_perm[k]);
             vec2_t* o = d.aux_out + b * d.aux_out_bs;
-            o[uint64_t(idx) * d.aux_out_es] = cscale(cadd(v, x0), d.scale);
-            if (k == 0) o[0] = cscale(__ldcg(&d.aux_in[2 * uint64_t(b) + 1]), d.scale);
+            o[uint64_t(idx) * d.aux_out_es] = cscale(v, d.scale);
+            if (k == 0) o[0] = cscale(__ldcg(&d.aux_in[b]), d.scale);
             break;
         }
         default:
@@ -775,7 +777,18 @@ __device__ __forceinline__ void fused_pass(const PassDesc& d, const InnerStep& s
     const uint32_t items = d.C * m;
     const bool cfast = (sio == IO_GLOBAL) ? (d.load_mode == MODE_LANE)
                                           : ((dio == IO_GLOBAL) ? (d.store_mode == MODE_LANE) : false);
+#if defined(KFFT_HALF_SCALAR)
     for (uint32_t it = threadIdx.x; it < items; it += blockDim.x) {
+#else
+    // d.inplace (one butterfly a thread, `src` and `dst` one buffer): every
+    // thread meets the barrier between the reads and the writes, those
+    // without a butterfly on a copy of the last one that they do not store
+    const bool exchange = d.inplace && sio == IO_SMEM && dio == IO_SMEM;
+    for (uint32_t i0 = 0; i0 < items; i0 += blockDim.x) {
+        const bool act = i0 + threadIdx.x < items;
+        if (!act && !exchange) break;
+        const uint32_t it = act ? i0 + threadIdx.x : items - 1;
+#endif
         uint32_t c, jj;
         if (cfast) {
             jj = fdiv(it, d.div_C);
@@ -813,6 +826,10 @@ __device__ __forceinline__ void fused_pass(const PassDesc& d, const InnerStep& s
         if (st.ns > 1) apply_inner_twiddles<P>(v, d.tw_inner, kk * st.twstride);
         dft<P, INV>(v);
         const uint32_t ob = blk * st.ns * P + kk;
+#if !defined(KFFT_HALF_SCALAR)
+        if (exchange) __syncthreads();
+        if (!act) break;
+#endif
         if (dio == IO_SMEM) {
 #pragma unroll
             for (int q = 0; q < P; ++q) dst[c * d.lane_stride + pad(ob + q * st.ns)] = v[q];
@@ -1436,8 +1453,8 @@ __device__ __forceinline__ void tile_body_reg(const PassDesc& d, const PassExtra
         return;
     }
     vec2_t* bufA = sm;
-    vec2_t* bufB = sm + d.C * d.lane_stride + 1;
 #if defined(KFFT_HALF_SCALAR)
+    vec2_t* bufB = sm + d.C * d.lane_stride + 1;
     if constexpr (SPEC) switch (d.spec) {
         case 4: tile_body_spec<16, INV>(d, lane0, total, bufA, bufB); return;
         case 5: tile_body_spec<32, INV>(d, lane0, total, bufA, bufB); return;
@@ -1450,6 +1467,8 @@ __device__ __forceinline__ void tile_body_reg(const PassDesc& d, const PassExtra
         case 12: tile_body_spec<4096, INV>(d, lane0, total, bufA, bufB); return;
         default: break;
     }
+#else
+    vec2_t* bufB = d.inplace ? sm : sm + d.C * d.lane_stride + 1;
 #endif
     const vec2_t* src = nullptr;
 #if defined(KFFT_HALF_SCALAR)

@@ -9,6 +9,7 @@
 
 namespace kfft {
 
+#if defined(KFFT_HALF_SCALAR)
 template <bool INV>
 __global__ void __launch_bounds__(kPassThreads, KFFT_REG_MINBLOCKS) k_pass_reg(const __grid_constant__ PassDesc d,
                                                               const __grid_constant__ PassExtra x) {
@@ -17,7 +18,6 @@ __global__ void __launch_bounds__(kPassThreads, KFFT_REG_MINBLOCKS) k_pass_reg(c
     tile_body_reg<INV, false>(d, x, blockIdx.x, reinterpret_cast<vec2_t*>(smem_raw));
 }
 
-#if defined(KFFT_HALF_SCALAR)
 // FP32 power-of-two passes, one kernel per pass length R so each kernel holds
 // only its own body (a small instruction footprint):
 // * k_pass_pipe: a plain prologue and more tiles than fit the GPU at once: a
@@ -199,6 +199,7 @@ bool take_wait_failures(cudaStream_t st) {
 #endif
 }
 
+#if defined(KFFT_HALF_SCALAR)
 void launch_pass_reg(const PassDesc& d, const PassExtra& x, cudaStream_t st) {
     // one-time shared-memory limit of the generic kernels (thread-safe; a
     // failure is reported on every call)
@@ -217,7 +218,6 @@ void launch_pass_reg(const PassDesc& d, const PassExtra& x, cudaStream_t st) {
         note_cuda_error(configured);
         return;
     }
-#if defined(KFFT_HALF_SCALAR)
     if (d.spec && d.threads == kPassThreads) {
         const bool inv = d.inv != 0;
         // one pass over whole contiguous sequences, 16-byte aligned: the
@@ -279,12 +279,12 @@ void launch_pass_reg(const PassDesc& d, const PassExtra& x, cudaStream_t st) {
             return;
         }
     }
-#endif
     if (d.inv) k_pass_reg<true><<<d.tiles, d.threads, d.smem_bytes, st>>>(d, x);
     else k_pass_reg<false><<<d.tiles, d.threads, d.smem_bytes, st>>>(d, x);
     note_cuda_error(cudaGetLastError());
     count_launch();
 }
+#endif
 
 }  // namespace kfft
 

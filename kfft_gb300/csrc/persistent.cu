@@ -2,6 +2,7 @@
 // queue of (pass, tile) items ordered by dependency level, with bounded waits
 // on per-pass tile counters (a wait that gives up sets an error word).
 #include "fft_device.cuh"
+#include "fx_spec.cuh"
 
 #include <mutex>
 
@@ -78,8 +79,27 @@ __device__ __forceinline__ void stage_desc(const PassDesc* __restrict__ descs, u
 
 __device__ __forceinline__ void run_item(const PassDesc& d, const PassExtra& x, uint32_t tile,
                                          vec2_t* buf) {
+#if !defined(KFFT_HALF_SCALAR)
+    unsigned char* smem = reinterpret_cast<unsigned char*>(buf);
+    bool ok = false;
+    if (d.fx) {
+        switch (d.spec) {
+            case 4: ok = fx_spec_tile<16>(d, tile, smem); break;
+            case 5: ok = fx_spec_tile<32>(d, tile, smem); break;
+            case 6: ok = fx_spec_tile<64>(d, tile, smem); break;
+            case 7: ok = fx_spec_tile<128>(d, tile, smem); break;
+            case 8: ok = fx_spec_tile<256>(d, tile, smem); break;
+            case 9: ok = fx_spec_tile<512>(d, tile, smem); break;
+            case 10: ok = fx_spec_tile<1024>(d, tile, smem); break;
+            case 11: ok = fx_spec_tile<2048>(d, tile, smem); break;
+            default: ok = fx_tile(d, x, tile, smem); break;
+        }
+    }
+    if (!ok) fp64_tile(d, x, tile, smem);
+#else
     if (d.inv) tile_body_reg<true, true, false>(d, x, tile, buf);
     else tile_body_reg<false, true, false>(d, x, tile, buf);
+#endif
 }
 
 __global__ void __launch_bounds__(KFFT_QUEUE_THREADS, KFFT_QUEUE_MINBLOCKS) k_persistent(

@@ -222,6 +222,9 @@ static bool build_direct(FftPlan* P, DeviceArena& arena, cudaStream_t st) {
     if (Rs.empty()) return false;
     if (V.reverse) std::reverse(Rs.begin(), Rs.end());
     std::map<uint32_t, const vec2_t*> inner;
+#if !defined(KFFT_HALF_SCALAR)
+    std::map<uint32_t, const FxTw*> fx_inner;
+#endif
     uint32_t Ns = 1;
     for (uint32_t R : Rs) {
         PassSpec s;
@@ -235,8 +238,17 @@ static bool build_direct(FftPlan* P, DeviceArena& arena, cudaStream_t st) {
             if (!t) return false;
             gen_twiddles(t, R, 1, R, P->sign, st);
             it = inner.emplace(R, t).first;
+#if !defined(KFFT_HALF_SCALAR)
+            FxTw* f = static_cast<FxTw*>(arena.alloc(sizeof(FxTw) * R));
+            if (!f) return false;
+            gen_fx_twiddles(f, R, 1, R, st);
+            fx_inner[R] = f;
+#endif
         }
         s.tw_inner = it->second;
+#if !defined(KFFT_HALF_SCALAR)
+        s.fx_inner = fx_inner[R];
+#endif
         P->passes.push_back(s);
         Ns *= R;
     }
@@ -251,6 +263,15 @@ static bool build_direct(FftPlan* P, DeviceArena& arena, cudaStream_t st) {
         if (!lo || !hi) return false;
         gen_twiddles(lo, nlo, 1, N, P->sign, st);
         gen_twiddles(hi, nhi, uint64_t(nlo), N, P->sign, st);
+#if !defined(KFFT_HALF_SCALAR)
+        FxTw* flo = static_cast<FxTw*>(arena.alloc(sizeof(FxTw) * nlo));
+        FxTw* fhi = static_cast<FxTw*>(arena.alloc(sizeof(FxTw) * nhi));
+        if (!flo || !fhi) return false;
+        gen_fx_twiddles(flo, nlo, 1, N, st);
+        gen_fx_twiddles(fhi, nhi, uint64_t(nlo), N, st);
+        P->fx_lo = flo;
+        P->fx_hi = fhi;
+#endif
         P->tw_lo = lo;
         P->tw_hi = hi;
         P->tw_shift = shift;
@@ -304,6 +325,30 @@ PlanVariant plan_variant(uint32_t index) {
         default: break;
     }
     return v;
+}
+
+// The two-limb forms of a Rader or Bluestein plan's tables (double build).
+static bool fx_tables(FftPlan* P, DeviceArena& arena, int sign, cudaStream_t st) {
+#if defined(KFFT_HALF_SCALAR)
+    (void)P, (void)arena, (void)sign, (void)st;
+    return true;
+#else
+    FxTw* f = static_cast<FxTw*>(arena.alloc(sizeof(FxTw) * P->L));
+    int32_t* e = static_cast<int32_t*>(arena.alloc(sizeof(int32_t)));
+    if (!f || !e) return false;
+    gen_fx_spectrum(f, P->spectrum, P->L, e, st);
+    P->fx_spectrum = f;
+    if (P->chirp) {
+        FxTw* c = static_cast<FxTw*>(arena.alloc(sizeof(FxTw) * P->N));
+        if (!c) return false;
+        gen_fx_chirp(c, P->N, P->N, sign, st);
+        P->fx_chirp = c;
+    }
+    cudaMemcpyAsync(&P->fx_spectrum_e, e, sizeof(int32_t), cudaMemcpyDeviceToHost, st);
+    const cudaError_t r = cudaStreamSynchronize(st);
+    if (r != cudaSuccess) note_cuda_error(r);
+    return r == cudaSuccess;
+#endif
 }
 
 // 1: a Bluestein plan sizes its convolution for the pass limits of its own
@@ -372,6 +417,10 @@ FftPlan* make_plan(uint32_t N, int sign, DeviceArena& arena, cudaStream_t st,
         }
         scale_table(spec, L, 1.0 / double(L), st);
         P->spectrum = spec;
+        if (!fx_tables(P, arena, sign, st)) {
+            delete P;
+            return nullptr;
+        }
         return P;
     }
     // ---- Bluestein: X_k = c_k sum_n (x_n c_n) conj(c_{k-n}) --------------------
@@ -410,6 +459,10 @@ FftPlan* make_plan(uint32_t N, int sign, DeviceArena& arena, cudaStream_t st,
     scale_table(spec, uint32_t(M), 1.0 / double(M), st);
     P->chirp = chirp;
     P->spectrum = spec;
+    if (!fx_tables(P, arena, sign, st)) {
+        delete P;
+        return nullptr;
+    }
     return P;
 }
 
@@ -459,7 +512,7 @@ size_t workspace_bytes(const FftPlan& p, uint32_t batch) {
         return 0;
     }
     size_t a = round256(sizeof(vec2_t) * size_t(p.L) * batch);
-    size_t extra = (p.method == METHOD_RADER) ? round256(sizeof(vec2_t) * 2 * size_t(batch)) : 0;
+    size_t extra = (p.method == METHOD_RADER) ? round256(sizeof(vec2_t) * size_t(batch)) : 0;
     return a + extra + std::max(workspace_bytes(*p.sub_fwd, batch), workspace_bytes(*p.sub_inv, batch));
 }
 
@@ -475,6 +528,11 @@ struct Fuse {
     vec2_t* aux_out = nullptr;
     uint64_t aux_in_bs = 0, aux_out_bs = 0;
     uint32_t aux_out_es = 1;
+#if !defined(KFFT_HALF_SCALAR)
+    const FxTw* fx_pro = nullptr;
+    const FxTw* fx_epi = nullptr;
+    int32_t fx_epi_e = 0;
+#endif
 };
 
 static PassDesc make_desc(const FftPlan& P, size_t pi, const vec2_t* in, const Layout& lin,
@@ -557,7 +615,14 @@ static PassDesc make_desc(const FftPlan& P, size_t pi, const vec2_t* in, const L
     // (FP32 only: in FP64 its fully unrolled stages spill and the FP64 pipe,
     // not index arithmetic, bounds the pass)
     d.spec = 0;
-#if defined(KFFT_HALF_SCALAR)
+#if !defined(KFFT_HALF_SCALAR)
+    // power-of-two passes run fx_spec_tile: 8 points a thread
+    if (d.regmode && s.R >= 16 && s.R <= 4096 && (s.R & (s.R - 1)) == 0) {
+        uint32_t l = 0;
+        while ((1u << l) < s.R) ++l;
+        d.spec = uint8_t(l);
+    }
+#else
     if (d.regmode && !d.tc && s.R >= 16 && s.R <= 4096 && (s.R & (s.R - 1)) == 0) {
         uint32_t l = 0;
         while ((1u << l) < s.R) ++l;
@@ -569,10 +634,24 @@ static PassDesc make_desc(const FftPlan& P, size_t pi, const vec2_t* in, const L
     uint32_t elems = C * s.R;
     if (d.regmode) {
         d.threads = kPassThreads;
+#if defined(KFFT_HALF_SCALAR)
         const uint32_t nbuf = s.radices.size() >= 3 ? 2u : (s.radices.size() == 2 ? 1u : 0u);
+#else
+        // one buffer where no stage has more than one butterfly a thread
+        d.inplace = 1;
+        for (uint8_t r : s.radices)
+            if (!d.spec && uint64_t(C) * (s.R / r) > kPassThreads) d.inplace = 0;
+        const uint32_t nbuf = d.inplace ? 1u : 2u;
+        d.fx = d.nrad > 0 && elems <= kFxElems * kPassThreads ? 1 : 0;
+        if (d.spec) d.threads = std::max<uint32_t>(32, (elems / 8 + 31) / 32 * 32);
+#endif
         d.lane_stride = spec_lane_stride(s.R, C, d.load_mode == MODE_LANE,
                                          d.store_mode == MODE_LANE, kPassThreads);
         d.smem_bytes = nbuf * (C * d.lane_stride + 1u) * uint32_t(sizeof(vec2_t));
+#if !defined(KFFT_HALF_SCALAR)
+        d.fx_words = d.smem_bytes;
+        d.smem_bytes += std::max<uint32_t>(d.nrad, kFxRows) * C * uint32_t(sizeof(uint32_t));
+#endif
     } else {
         uint32_t t = (elems + 7) / 8;
         t = (t + 31) / 32 * 32;
@@ -590,6 +669,22 @@ static PassDesc make_desc(const FftPlan& P, size_t pi, const vec2_t* in, const L
     d.tw_shift = P.tw_shift;
     d.tw_mul = d.lanes_j / s.Ns;
     d.scale = scale;
+#if !defined(KFFT_HALF_SCALAR)
+    d.fx_inner = s.fx_inner;
+    d.fx_lo = P.fx_lo;
+    d.fx_hi = P.fx_hi;
+    {
+        // scale = f * 2^e, f in [1/2, 1): a power of two needs no product
+        int e = 0;
+        const double f = std::frexp(scale, &e);
+        d.fx_scale_e = f == 0.5 ? e - 1 : e;
+        if (f != 0.5) {
+            const int64_t v = int64_t(std::ldexp(f, 62));
+            d.fx_scale_l = int32_t(uint32_t(uint64_t(v)));
+            d.fx_scale_h = int32_t((v - d.fx_scale_l) >> 32);
+        }
+    }
+#endif
     return d;
 }
 
@@ -604,6 +699,9 @@ static void apply_fuse(PassDesc& d, const Fuse& f, bool first, bool last) {
         d.pro_tab = f.pro_tab;
         d.pro_perm = f.pro_perm;
         d.pro_bound = f.pro_bound;
+#if !defined(KFFT_HALF_SCALAR)
+        d.fx_pro = f.fx_pro;
+#endif
     }
     if (last) {
         d.epi_op = f.epi_op;
@@ -615,6 +713,10 @@ static void apply_fuse(PassDesc& d, const Fuse& f, bool first, bool last) {
         d.aux_in_bs = f.aux_in_bs;
         d.aux_out_bs = f.aux_out_bs;
         d.aux_out_es = f.aux_out_es;
+#if !defined(KFFT_HALF_SCALAR)
+        d.fx_epi = f.fx_epi;
+        d.fx_epi_e = f.fx_epi_e;
+#endif
     }
 }
 
@@ -680,6 +782,11 @@ bool build_passes(const FftPlan& P, const vec2_t* in, const Layout& lin, vec2_t*
         ff.pro_bound = P.N;
         ff.epi_op = EPI_MUL;
         ff.epi_tab = P.spectrum;
+#if !defined(KFFT_HALF_SCALAR)
+        ff.fx_pro = P.fx_chirp;
+        ff.fx_epi = P.fx_spectrum;
+        ff.fx_epi_e = P.fx_spectrum_e;
+#endif
         Layout lx = lin;  // the input seen as length-L sequences with the caller's strides
         const size_t mark = ws.used;
         if (!build_direct_passes(*P.sub_fwd, in, lx, A, la, real_t(1), ff, ws, descs)) return false;
@@ -688,26 +795,33 @@ bool build_passes(const FftPlan& P, const vec2_t* in, const Layout& lin, vec2_t*
         fi.epi_op = EPI_CHIRP;
         fi.epi_tab = P.chirp;
         fi.epi_bound = P.N;
+#if !defined(KFFT_HALF_SCALAR)
+        fi.fx_epi = P.fx_chirp;
+#endif
         return build_direct_passes(*P.sub_inv, A, la, out, lout, scale, fi, ws, descs);
     }
     // Rader
-    vec2_t* pairs = ws.take(size_t(2) * B);
-    if (!pairs) return false;
+    vec2_t* sums = ws.take(size_t(B));  // X_0 of each sequence
+    if (!sums) return false;
     Fuse ff;
     ff.pro_op = PRO_GATHER;
     ff.pro_perm = P.gperm;
     ff.epi_op = EPI_RADER_FWD;
     ff.epi_tab = P.spectrum;
+#if !defined(KFFT_HALF_SCALAR)
+    ff.fx_epi = P.fx_spectrum;
+    ff.fx_epi_e = P.fx_spectrum_e;
+#endif
     ff.aux_in = in;
     ff.aux_in_bs = lin.bs;
-    ff.aux_out = pairs;
+    ff.aux_out = sums;
     const size_t mark = ws.used;
     if (!build_direct_passes(*P.sub_fwd, in, lin, A, la, real_t(1), ff, ws, descs)) return false;
     ws.used = mark;  // the inverse reuses the forward's scratch (stream ordered)
     Fuse fi;
     fi.epi_op = EPI_RADER_INV;
     fi.epi_perm = P.iperm;
-    fi.aux_in = pairs;
+    fi.aux_in = sums;
     fi.aux_out = out;
     fi.aux_out_bs = lout.bs;
     fi.aux_out_es = lout.es;
