@@ -57,12 +57,16 @@ struct FastDiv {
 struct alignas(16) FxTw {
     int32_t rh, rl, ih, il;
 };
-// elements a thread of a fixed-point tile holds at most
-constexpr uint32_t kFxElems = 16;
+// bytes a lane's table entry takes (FxLane in fx_tile.cuh)
+constexpr uint32_t kFxLaneBytes = 32;
+// butterflies of radix P a thread of a run-time tile runs side by side
+constexpr uint32_t fx_group(uint32_t P) { return P == 2 ? 4 : (P == 3 ? 3 : (P <= 6 ? 2 : 1)); }
 // rows of lane words a fixed-point tile has at least (one a stage)
 constexpr uint32_t kFxRows = 4;
 // threads of a full power-of-two fixed-point tile (8 points each)
 constexpr uint32_t kFxSpecThreads = 512;
+// most threads of a run-time fixed-point tile
+constexpr uint32_t kFxWideThreads = 512;
 
 enum : uint8_t { MODE_LANE = 0, MODE_ELEM = 1 };
 enum : uint8_t { ORDER_J = 0, ORDER_B = 1 };
@@ -129,7 +133,8 @@ struct PassDesc {
     // fixed-point tile (fx_tile.cuh): forward tables in two-limb form
     uint8_t fx;             // the tile runs in fixed point
     uint8_t inplace;        // three or more stages of one butterfly a thread: one exchange buffer
-    uint32_t fx_words;      // byte offset of the lane words in shared memory
+    uint32_t fx_words;      // byte offsets of the lane words and the lane table in shared memory
+    uint32_t fx_lanes;
     const FxTw* fx_inner;   // tw_inner's forward twiddles
     const FxTw* fx_lo;      // tw_lo's and tw_hi's
     const FxTw* fx_hi;
@@ -138,6 +143,7 @@ struct PassDesc {
     int32_t fx_epi_e;
     int32_t fx_scale_h, fx_scale_l;  // scale = 2^fx_scale_e, times these limbs / 2^62 unless zero
     int32_t fx_scale_e;
+    int32_t fx_one;         // 1 (a factor the compiler does not know)
 #endif
 };
 
@@ -230,6 +236,15 @@ struct PassSpec {
 
 struct DeviceArena;  // device memory owned by a plan tree
 
+// threads per CTA of the queue kernel (its tile bodies stride over the
+// CTA's threads, whatever their number).  Uneven FP32 batch: 256 threads,
+// 2048-point tiles, 4 CTAs per SM 8.85 ms; 128 threads, 1024-point tiles,
+// 256-point passes, 8 CTAs 9.05 ms (6 CTAs 10.17); 512 threads,
+// 4096-point tiles, 2 CTAs 9.47 ms with 1024-point passes, 10.10 with 512.
+#ifndef KFFT_QUEUE_THREADS
+#define KFFT_QUEUE_THREADS 256
+#endif
+
 // Planner knobs one plan variant fixes (the tuner's search space).
 // Largest pass length of variant 0's multi-pass splits (a build-time knob for
 // sweeps; variants 1 and 2 lower it to 512 and 256).
@@ -243,6 +258,7 @@ struct PlanVariant {
     uint32_t single_div = 1;     // divisor on the default lanes of single-pass tiles
     uint32_t single_cap = 4096;  // longest length run as one fused pass
     uint32_t tile_cap = kRegTile;  // most points per register tile
+    uint32_t fx_threads = 512;   // most threads of a fixed-point tile (double build)
     bool reverse = false;        // multi-pass splits run longest pass last
     bool no_rader = false;       // primes through Bluestein even where Rader applies
     bool no_fused = false;       // shared-memory ping-pong tiles only

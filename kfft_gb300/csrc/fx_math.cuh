@@ -118,9 +118,11 @@ __device__ __forceinline__ fx_t fx_mulcc(int32_t a) {
     asm("mul.wide.s32 %0, %1, %2;" : "=l"(r) : "r"(a), "n"(B));
     return r;
 }
-// c + the high word of v, sign extended (one mad.wide)
-__device__ __forceinline__ fx_t fx_add_high(fx_t v, fx_t c) {
-    return fx_madc<1>(int32_t(v >> 32), c);
+// c + the high word of v, sign extended: one mad.wide by `one`, a 1 that the
+// compiler does not know (PassDesc::fx_one; a known 1 becomes three
+// instructions on the ALU pipe, the busiest one here)
+__device__ __forceinline__ fx_t fx_add_high(fx_t v, fx_t c, int32_t one) {
+    return fx_mad(int32_t(v >> 32), one, c);
 }
 // signed limbs of a value: v = h * 2^32 + l, l as a signed word
 struct FxLimbs {
@@ -134,7 +136,7 @@ __device__ __forceinline__ FxLimbs fx_limbs(fx_t v) {
 }
 
 // a * w / 4 for a twiddle w (|w| <= 1), |a| <= 2^62.5
-__device__ __forceinline__ cfx_t fx_cmul(cfx_t a, const FxTw& w) {
+__device__ __forceinline__ cfx_t fx_cmul(cfx_t a, const FxTw& w, int32_t one) {
     const FxLimbs x = fx_limbs(a.x), y = fx_limbs(a.y);
     const int32_t nih = -w.ih, nil = -w.il;
     fx_t cr = fx_mul(x.h, w.rl);
@@ -146,13 +148,13 @@ __device__ __forceinline__ cfx_t fx_cmul(cfx_t a, const FxTw& w) {
     ci = fx_mad(y.h, w.rl, ci);
     ci = fx_mad(y.l, w.rh, ci);
     cfx_t r;
-    r.x = fx_add_high(cr, fx_mad(y.h, nih, fx_mul(x.h, w.rh)));
-    r.y = fx_add_high(ci, fx_mad(y.h, w.rh, fx_mul(x.h, w.ih)));
+    r.x = fx_add_high(cr, fx_mad(y.h, nih, fx_mul(x.h, w.rh)), one);
+    r.y = fx_add_high(ci, fx_mad(y.h, w.rh, fx_mul(x.h, w.ih)), one);
     return r;
 }
 
 // the twiddle a * w of two twiddles
-__device__ __forceinline__ FxTw fx_tw_mul(const FxTw& a, const FxTw& w) {
+__device__ __forceinline__ FxTw fx_tw_mul(const FxTw& a, const FxTw& w, int32_t one) {
     const int32_t nih = -w.ih, nil = -w.il;
     fx_t cr = fx_mul(a.rh, w.rl);
     cr = fx_mad(a.rl, w.rh, cr);
@@ -162,8 +164,8 @@ __device__ __forceinline__ FxTw fx_tw_mul(const FxTw& a, const FxTw& w) {
     ci = fx_mad(a.rl, w.ih, ci);
     ci = fx_mad(a.ih, w.rl, ci);
     ci = fx_mad(a.il, w.rh, ci);
-    const fx_t re = fx_add_high(cr, fx_mad(a.ih, nih, fx_mul(a.rh, w.rh))) << 2;
-    const fx_t im = fx_add_high(ci, fx_mad(a.ih, w.rh, fx_mul(a.rh, w.ih))) << 2;
+    const fx_t re = fx_add_high(cr, fx_mad(a.ih, nih, fx_mul(a.rh, w.rh)), one) << 2;
+    const fx_t im = fx_add_high(ci, fx_mad(a.ih, w.rh, fx_mul(a.rh, w.ih)), one) << 2;
     FxTw r;
     const FxLimbs p = fx_limbs(re), q = fx_limbs(im);
     r.rh = p.h;
@@ -173,11 +175,12 @@ __device__ __forceinline__ FxTw fx_tw_mul(const FxTw& a, const FxTw& w) {
     return r;
 }
 
-// x times the constant N + F / 2^64 (|F| <= 2^63, N in -1, 0, 1): exact to
-// about one unit, no rescaling
-template <int N, fx_t F>
-__device__ __forceinline__ fx_t fx_mulc(fx_t x, FxLimbs l) {
-    fx_t acc = N == 1 ? x : (N == -1 ? -x : 0);
+// x times the constant N + F / 2^64 (|F| <= 2^63, N in -1, 0, 1), or with
+// ACC that added to `acc`: exact to about one unit, no rescaling
+template <int N, fx_t F, bool ACC = false>
+__device__ __forceinline__ fx_t fx_mulc(fx_t x, FxLimbs l, int32_t one, fx_t acc = 0) {
+    if (N == 1) acc = ACC ? acc + x : x;
+    if (N == -1) acc = ACC ? acc - x : -x;
     if constexpr (F == 0) {
         return acc;
     } else if constexpr (F == INT64_MIN) {
@@ -185,9 +188,9 @@ __device__ __forceinline__ fx_t fx_mulc(fx_t x, FxLimbs l) {
     } else {
         constexpr int32_t fl = fx_lo(F), fh = fx_hi(F);
         const fx_t cross = fx_madc<fh>(l.l, fx_mulcc<fl>(l.h));
-        if constexpr (N == 0) acc = fx_mulcc<fh>(l.h);
+        if constexpr (N == 0 && !ACC) acc = fx_mulcc<fh>(l.h);
         else acc = fx_madc<fh>(l.h, acc);
-        return fx_add_high(cross, acc);
+        return fx_add_high(cross, acc, one);
     }
 }
 
@@ -215,7 +218,7 @@ constexpr fx_t fx_const_f(fx_t v) { return (v - fx_t(fx_const_n(v)) * kFxOne) * 
 
 // a * W_P^E (W = exp(-2 pi i / P)), E modulo P
 template <int P, int E>
-__device__ __forceinline__ cfx_t fx_wmul(cfx_t a) {
+__device__ __forceinline__ cfx_t fx_wmul(cfx_t a, int32_t one) {
     constexpr int e = ((E % P) + P) % P;
     if constexpr (e == 0) {
         return a;
@@ -230,7 +233,7 @@ __device__ __forceinline__ cfx_t fx_wmul(cfx_t a) {
         constexpr int rn = fx_const_n(r);
         constexpr fx_t rf = fx_const_f(r);
         const fx_t s = a.x + a.y, t = a.y - a.x;
-        const fx_t p = fx_mulc<rn, rf>(s, fx_limbs(s)), m = fx_mulc<rn, rf>(t, fx_limbs(t));
+        const fx_t p = fx_mulc<rn, rf>(s, fx_limbs(s), one), m = fx_mulc<rn, rf>(t, fx_limbs(t), one);
         constexpr int o = (8 * e) / P;
         if constexpr (o == 1) return cfx_t{p, m};
         else if constexpr (o == 3) return cfx_t{m, -p};
@@ -242,8 +245,8 @@ __device__ __forceinline__ cfx_t fx_wmul(cfx_t a) {
         constexpr fx_t cf = fx_const_f(c), sf = fx_const_f(s), nsf = fx_const_f(-s);
         const FxLimbs x = fx_limbs(a.x), y = fx_limbs(a.y);
         // (x + i y)(c - i s)
-        return {fx_mulc<cn, cf>(a.x, x) + fx_mulc<sn, sf>(a.y, y),
-                fx_mulc<cn, cf>(a.y, y) + fx_mulc<nsn, nsf>(a.x, x)};
+        return {fx_mulc<sn, sf, true>(a.y, y, one, fx_mulc<cn, cf>(a.x, x, one)),
+                fx_mulc<nsn, nsf, true>(a.x, x, one, fx_mulc<cn, cf>(a.y, y, one))};
     }
 }
 
@@ -265,7 +268,7 @@ __device__ __forceinline__ void fx_for(F&& f) {
 }
 
 template <int P>
-__device__ __forceinline__ void fx_dft_odd(cfx_t* v) {
+__device__ __forceinline__ void fx_dft_odd(cfx_t* v, int32_t one) {
     constexpr int H = (P - 1) / 2;
     cfx_t s[H], d[H];
     const cfx_t x0 = v[0];
@@ -284,10 +287,10 @@ __device__ __forceinline__ void fx_dft_odd(cfx_t* v) {
             constexpr fx_t c = fx_const62(long(n) * K, P, false), si = fx_const62(long(n) * K, P, true);
             constexpr int cn = fx_const_n(c), sn = fx_const_n(si);
             constexpr fx_t cf = fx_const_f(c), sf = fx_const_f(si);
-            a.x += fx_mulc<cn, cf>(s[n - 1].x, fx_limbs(s[n - 1].x));
-            a.y += fx_mulc<cn, cf>(s[n - 1].y, fx_limbs(s[n - 1].y));
-            b.x += fx_mulc<sn, sf>(d[n - 1].x, fx_limbs(d[n - 1].x));
-            b.y += fx_mulc<sn, sf>(d[n - 1].y, fx_limbs(d[n - 1].y));
+            a.x = fx_mulc<cn, cf, true>(s[n - 1].x, fx_limbs(s[n - 1].x), one, a.x);
+            a.y = fx_mulc<cn, cf, true>(s[n - 1].y, fx_limbs(s[n - 1].y), one, a.y);
+            b.x = fx_mulc<sn, sf, true>(d[n - 1].x, fx_limbs(d[n - 1].x), one, b.x);
+            b.y = fx_mulc<sn, sf, true>(d[n - 1].y, fx_limbs(d[n - 1].y), one, b.y);
         });
         v[K] = {a.x + b.y, a.y - b.x};      // a - i b
         v[P - K] = {a.x - b.y, a.y + b.x};  // a + i b
@@ -303,11 +306,11 @@ constexpr int fx_modinv(int a, int m) {
 }
 
 template <int P>
-__device__ __forceinline__ void fx_dft(cfx_t* v);
+__device__ __forceinline__ void fx_dft(cfx_t* v, int32_t one);
 
 // P = A * B: Good-Thomas for coprime factors, else Cooley-Tukey
 template <int A, int B>
-__device__ __forceinline__ void fx_dft_composite(cfx_t* v) {
+__device__ __forceinline__ void fx_dft_composite(cfx_t* v, int32_t one) {
     constexpr int P = A * B;
     constexpr bool kPfa = fx_gcd(A, B) == 1;
     cfx_t t[P];
@@ -318,11 +321,11 @@ __device__ __forceinline__ void fx_dft_composite(cfx_t* v) {
             constexpr int n1 = decltype(n1c)::value;
             a[n1] = v[kPfa ? (B * n1 + A * n2) % P : B * n1 + n2];
         });
-        fx_dft<A>(a);
+        fx_dft<A>(a, one);
         fx_for<0, A>([&](auto k1c) {
             constexpr int k1 = decltype(k1c)::value;
             if constexpr (kPfa) t[n2 * A + k1] = a[k1];
-            else t[n2 * A + k1] = fx_wmul<P, n2 * k1>(a[k1]);
+            else t[n2 * A + k1] = fx_wmul<P, n2 * k1>(a[k1], one);
         });
     });
     fx_for<0, A>([&](auto k1c) {
@@ -332,7 +335,7 @@ __device__ __forceinline__ void fx_dft_composite(cfx_t* v) {
             constexpr int n2 = decltype(n2c)::value;
             b[n2] = t[n2 * A + k1];
         });
-        fx_dft<B>(b);
+        fx_dft<B>(b, one);
         fx_for<0, B>([&](auto k2c) {
             constexpr int k2 = decltype(k2c)::value;
             v[kPfa ? (B * fx_modinv(B % A, A) * k1 + A * fx_modinv(A % B, B) * k2) % P : k1 + A * k2] =
@@ -342,21 +345,21 @@ __device__ __forceinline__ void fx_dft_composite(cfx_t* v) {
 }
 
 template <int P>
-__device__ __forceinline__ void fx_dft(cfx_t* v) {
+__device__ __forceinline__ void fx_dft(cfx_t* v, int32_t one) {
     if constexpr (P == 2) {
         const cfx_t t = v[0];
         v[0] = fx_add(t, v[1]);
         v[1] = fx_sub(t, v[1]);
     } else if constexpr (P == 4) fx_dft4(v[0], v[1], v[2], v[3]);
-    else if constexpr (P == 8) fx_dft_composite<2, 4>(v);
-    else if constexpr (P == 16) fx_dft_composite<4, 4>(v);
-    else if constexpr (P == 6) fx_dft_composite<2, 3>(v);
-    else if constexpr (P == 9) fx_dft_composite<3, 3>(v);
-    else if constexpr (P == 10) fx_dft_composite<2, 5>(v);
-    else if constexpr (P == 12) fx_dft_composite<4, 3>(v);
-    else if constexpr (P == 14) fx_dft_composite<2, 7>(v);
-    else if constexpr (P == 15) fx_dft_composite<3, 5>(v);
-    else fx_dft_odd<P>(v);
+    else if constexpr (P == 8) fx_dft_composite<2, 4>(v, one);
+    else if constexpr (P == 16) fx_dft_composite<4, 4>(v, one);
+    else if constexpr (P == 6) fx_dft_composite<2, 3>(v, one);
+    else if constexpr (P == 9) fx_dft_composite<3, 3>(v, one);
+    else if constexpr (P == 10) fx_dft_composite<2, 5>(v, one);
+    else if constexpr (P == 12) fx_dft_composite<4, 3>(v, one);
+    else if constexpr (P == 14) fx_dft_composite<2, 7>(v, one);
+    else if constexpr (P == 15) fx_dft_composite<3, 5>(v, one);
+    else fx_dft_odd<P>(v, one);
 }
 
 // headroom bits a radix-P butterfly needs beyond a factor 4
@@ -371,27 +374,33 @@ constexpr __host__ __device__ int fx_room(int P) { return P <= 4 ? 0 : (P <= 8 ?
 __device__ __forceinline__ fx_t fx_from_double(double d, int emax, int top) {
     const uint32_t hi = uint32_t(__double2hiint(d)), lo = uint32_t(__double2loint(d));
     const int e = int((hi >> 20) & 0x7ffu);
-    const uint32_t mh = (hi & 0xfffffu) | 0x100000u;
-    const uint64_t m = ((uint64_t(mh) << 32) | lo) << 9;  // leading bit at 61
-    const int rs = min(emax - e + (61 - top), 63);
-    const fx_t v = fx_t(m >> rs);
+    // the significand, leading bit at 63
+    const uint64_t m = (uint64_t(__funnelshift_l(lo, hi, 11) | 0x80000000u) << 32) | (lo << 11);
+    fx_t v;  // (shr clamps: a shift of 64 or more leaves zero)
+    asm("shr.u64 %0, %1, %2;" : "=l"(v) : "l"(m), "r"(emax + (63 - top) - e));
     const fx_t s = fx_t(int32_t(hi) >> 31);
     return (v ^ s) - s;
 }
 
-// v * 2^(eb - 1085) rounded to a double (the result is normal or zero)
+// v * 2^(eb - 1085) rounded to a double (|v| < 2^63; the result is normal or zero)
 __device__ __forceinline__ double fx_to_double(fx_t v, int eb) {
-    const uint32_t sgn = uint32_t(v >> 32) & 0x80000000u;
+    const uint32_t sgn = uint32_t(uint64_t(v) >> 32) & 0x80000000u;
     uint64_t a = uint64_t(v < 0 ? -v : v);
     if (uint32_t(a >> 32) == 0) {  // a value far below its lane's largest
         if (a == 0) return 0.0;
-        a <<= 32;
-        eb -= 32;
+        if (uint32_t(a) >> 31) {  // keep the leading bit below 63
+            a <<= 31;
+            eb -= 31;
+        } else {
+            a <<= 32;
+            eb -= 32;
+        }
     }
     const int lz = __clz(int(uint32_t(a >> 32)));
-    a <<= lz;
-    const uint64_t r = (a >> 11) + ((a >> 10) & 1u) + (uint64_t(uint32_t(eb - lz)) << 52);
-    return __hiloint2double(int(uint32_t(r >> 32) | sgn), int(uint32_t(r)));
+    // the leading bit at 62, half a unit of the 53 bits added
+    const uint64_t r = ((a << (lz - 1)) + 0x200u) >> 10;
+    return __hiloint2double(int((uint32_t(r >> 32) + (uint32_t(eb - lz) << 20)) | sgn),
+                            int(uint32_t(r)));
 }
 #endif
 

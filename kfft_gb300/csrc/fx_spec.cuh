@@ -56,16 +56,16 @@ __device__ __forceinline__ void fx_spec_store(const PassDesc& d, uint32_t g, uin
             if (op == EPI_RADER_FWD && k == 0) {
                 const double2 x0 = __ldcg(&d.aux_in[b * d.aux_in_bs]);
                 d.aux_out[b] = cadd(x0, double2{fx_to_double(u.x, eb), fx_to_double(u.y, eb)});
-                u = fx_cmul(u, fx_tw_load(d.fx_epi));
+                u = fx_cmul(u, fx_tw_load(d.fx_epi), d.fx_one);
                 out[0] = cadd(x0, double2{fx_to_double(u.x, e_out), fx_to_double(u.y, e_out)});
                 continue;
             }
-            u = fx_cmul(u, fx_tw_load(&d.fx_epi[k]));
+            u = fx_cmul(u, fx_tw_load(&d.fx_epi[k]), d.fx_one);
         }
         if (sh) {
             const FxLimbs x = fx_limbs(u.x), y = fx_limbs(u.y);
-            u.x = fx_add_high(fx_mad(x.l, sh, fx_mul(x.h, sl)), fx_mul(x.h, sh));
-            u.y = fx_add_high(fx_mad(y.l, sh, fx_mul(y.h, sl)), fx_mul(y.h, sh));
+            u.x = fx_add_high(fx_mad(x.l, sh, fx_mul(x.h, sl)), fx_mul(x.h, sh), d.fx_one);
+            u.y = fx_add_high(fx_mad(y.l, sh, fx_mul(y.h, sl)), fx_mul(y.h, sh), d.fx_one);
         }
         double2 r = {fx_to_double(u.x, e_out), fx_to_double(u.y, e_out)};
         double2* o = out;
@@ -91,15 +91,12 @@ __device__ __forceinline__ void fx_spec_exchange(const PassDesc& d, cfx_t* buf, 
 #pragma unroll
     for (int g = 0; g < G; ++g) {
         const uint32_t it = threadIdx.x + g * blockDim.x;
-        uint32_t b = 0;
+        uint32_t b = it < items ? fx_bits<P>(v[g]) : 0u;
         if (it < items) {
             cfx_t* o = buf + c[g] * d.lane_stride;
             const uint32_t ob = jj[g] % NS + (jj[g] / NS) * (NS * P);
 #pragma unroll
-            for (int q = 0; q < P; ++q) {
-                o[pad(ob + q * NS)] = v[g][q];
-                b |= fx_bits(v[g][q]);
-            }
+            for (int q = 0; q < P; ++q) o[pad(ob + q * NS)] = v[g][q];
         }
         if (M % 32 == 0 && !lane_mode) {  // the warp's butterflies are all of one lane
             b = __reduce_or_sync(0xffffffffu, b);
@@ -150,8 +147,8 @@ __device__ __forceinline__ void fx_spec_later(const PassDesc& d, cfx_t* buf, uin
             const uint32_t step = (jj[g] % NS) * TWS;
             v[g][0] = {v[g][0].x >> 2, v[g][0].y >> 2};
 #pragma unroll
-            for (int q = 1; q < P; ++q) v[g][q] = fx_cmul(v[g][q], fx_tw_load(&tw[q * step]));
-            fx_dft<P>(v[g]);
+            for (int q = 1; q < P; ++q) v[g][q] = fx_cmul(v[g][q], fx_tw_load(&tw[q * step]), d.fx_one);
+            fx_dft<P>(v[g], d.fx_one);
         }
     }
     if constexpr (kLast) {
@@ -218,13 +215,18 @@ __device__ __forceinline__ bool fx_spec_tile(const PassDesc& d, uint32_t tile, u
     __syncthreads();  // the words are zero
 #pragma unroll
     for (int g = 0; g < G; ++g) {
-        uint32_t m = 0, low = 0;
+        // the largest magnitude word: of the negative values (the unsigned
+        // maximum) and of the others (the signed one)
+        uint32_t neg = 0, low = 0;
+        int pos = 0;
 #pragma unroll
         for (int q = 0; q < P; ++q) {
-            m = max(m, max(uint32_t(__double2hiint(raw[g][q].x)) & 0x7fffffffu,
-                           uint32_t(__double2hiint(raw[g][q].y)) & 0x7fffffffu));
+            const int x = __double2hiint(raw[g][q].x), y = __double2hiint(raw[g][q].y);
+            neg = __vimax3_u32(neg, uint32_t(x), uint32_t(y));
+            pos = __vimax3_s32(pos, x, y);
             low |= uint32_t(__double2loint(raw[g][q].x)) | uint32_t(__double2loint(raw[g][q].y));
         }
+        uint32_t m = max(neg & 0x7fffffffu, uint32_t(pos));
         if (m == 0 && low) m = 1;
         bad = bad || (m >> 20) >= kFxExpHigh || (m != 0 && (m >> 20) < kFxExpLow);
         if (M % 32 == 0 && !lane_mode) {
@@ -258,18 +260,18 @@ __device__ __forceinline__ bool fx_spec_tile(const PassDesc& d, uint32_t tile, u
                     const FxTw w = fx_outer(d, uint32_t(uint64_t(M) * k * d.tw_mul));
 #pragma unroll
                     for (int q = 0; q < P; ++q) {
-                        v[g][q] = fx_cmul(v[g][q], t);
-                        if (q + 1 < P) t = fx_tw_mul(t, w);
+                        v[g][q] = fx_cmul(v[g][q], t, d.fx_one);
+                        if (q + 1 < P) t = fx_tw_mul(t, w, d.fx_one);
                     }
                 } else {
 #pragma unroll
                     for (int q = 0; q < P; ++q) {
                         const uint32_t n = j + (jj[g] + q * M) * d.lanes_j;
-                        if (n < d.pro_bound) v[g][q] = fx_cmul(v[g][q], fx_tw_load(&d.fx_pro[n]));
+                        if (n < d.pro_bound) v[g][q] = fx_cmul(v[g][q], fx_tw_load(&d.fx_pro[n]), d.fx_one);
                     }
                 }
             }
-            fx_dft<P>(v[g]);
+            fx_dft<P>(v[g], d.fx_one);
         }
     }
     fx_spec_exchange<P, G, R, 1>(d, buf, words + d.C, c, jj, v, lane_mode);

@@ -27,8 +27,20 @@ __global__ void __launch_bounds__(kFxSpecThreads, 2) k_fx_spec(const __grid_cons
 }
 
 #if KFFT_FX_PART == 0
-__global__ void __launch_bounds__(kPassThreads, 2) k_pass_fx(const __grid_constant__ PassDesc d,
-                                                             const __grid_constant__ PassExtra x) {
+#ifndef KFFT_FX_BLOCKS
+#define KFFT_FX_BLOCKS 3
+#endif
+#ifndef KFFT_FX_WIDE_BLOCKS
+#define KFFT_FX_WIDE_BLOCKS 2
+#endif
+// Run-time tiles: 256 threads, three CTAs an SM (80 registers; 16384 x 1000
+// points 416 us, 502 with two CTAs, 408 with four, but 4096 x 4000 794 against
+// 837); tiles whose exchange in one buffer takes more threads (above 2048
+// points or so) two CTAs of up to 512 (4096 x 4000 494 us, 612 with one CTA of
+// 128 registers, 794 with two buffers and 256 threads).
+template <uint32_t T, int BLOCKS>
+__global__ void __launch_bounds__(T, BLOCKS) k_pass_fx(const __grid_constant__ PassDesc d,
+                                                       const __grid_constant__ PassExtra x) {
     extern __shared__ __align__(16) unsigned char smem_raw[];
     double_tile(d, x, blockIdx.x, smem_raw);
 }
@@ -51,7 +63,8 @@ void launch_pass_reg(const PassDesc& d, const PassExtra& x, cudaStream_t st) {
             if (s >= 4 && !v.f[s]) v.f[s] = fx_kernels_2(s);
             if (s >= 4 && !v.f[s]) v.f[s] = fx_kernels_3(s);
         }
-        v.f[0] = k_pass_fx;
+        v.f[0] = k_pass_fx<kPassThreads, KFFT_FX_BLOCKS>;
+        v.f[1] = k_pass_fx<kFxWideThreads, KFFT_FX_WIDE_BLOCKS>;
         for (FxKernel f : v.f) {
             if (!f) continue;
             const cudaError_t e = cudaFuncSetAttribute(
@@ -67,7 +80,7 @@ void launch_pass_reg(const PassDesc& d, const PassExtra& x, cudaStream_t st) {
         note_cuda_error(k.error);
         return;
     }
-    k.f[d.fx ? d.spec : 0]<<<d.tiles, d.threads, d.smem_bytes, st>>>(d, x);
+    k.f[d.fx && d.spec ? d.spec : (d.threads > kPassThreads ? 1 : 0)]<<<d.tiles, d.threads, d.smem_bytes, st>>>(d, x);
     note_cuda_error(cudaGetLastError());
     count_launch();
 }

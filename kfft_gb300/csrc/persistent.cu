@@ -15,23 +15,15 @@ namespace kfft {
 #define KFFT_QUEUE_RELEASE_ONE 1
 #endif
 // resident CTAs per SM of the queue kernel (its tiles are capped at 2048
-// points): four for FP32 (64 registers a thread), three for FP64 (80
-// registers and about 2 KB of spills a thread, yet 84.1 against 87.7 ms for
-// two on the FP64 uneven batch)
+// points): four for FP32 (64 registers a thread), three for the double build
+// (80 registers; 256 sequences of up to 2^18 points 0.89 ms, two CTAs 0.95,
+// four 0.97)
 #ifndef KFFT_QUEUE_MINBLOCKS
 #if defined(KFFT_HALF_SCALAR)
 #define KFFT_QUEUE_MINBLOCKS 4
 #else
 #define KFFT_QUEUE_MINBLOCKS 3
 #endif
-#endif
-// threads per CTA of the queue kernel (its tile bodies stride over the
-// CTA's threads, whatever their number).  Uneven FP32 batch: 256 threads,
-// 2048-point tiles, 4 CTAs per SM 8.85 ms; 128 threads, 1024-point tiles,
-// 256-point passes, 8 CTAs 9.05 ms (6 CTAs 10.17); 512 threads,
-// 4096-point tiles, 2 CTAs 9.47 ms with 1024-point passes, 10.10 with 512.
-#ifndef KFFT_QUEUE_THREADS
-#define KFFT_QUEUE_THREADS 256
 #endif
 // 1: each CTA claims its items two ahead and copies the next item's record
 // into shared memory while the current one runs; 0: one claim ahead, the

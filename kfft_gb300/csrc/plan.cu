@@ -617,7 +617,8 @@ static PassDesc make_desc(const FftPlan& P, size_t pi, const vec2_t* in, const L
     d.spec = 0;
 #if !defined(KFFT_HALF_SCALAR)
     // power-of-two passes run fx_spec_tile: 8 points a thread
-    if (d.regmode && s.R >= 16 && s.R <= 4096 && (s.R & (s.R - 1)) == 0) {
+    if (d.regmode && s.R >= 16 && s.R <= 4096 && (s.R & (s.R - 1)) == 0 &&
+        C * s.R <= 8 * P.var.fx_threads) {
         uint32_t l = 0;
         while ((1u << l) < s.R) ++l;
         d.spec = uint8_t(l);
@@ -637,12 +638,16 @@ static PassDesc make_desc(const FftPlan& P, size_t pi, const vec2_t* in, const L
 #if defined(KFFT_HALF_SCALAR)
         const uint32_t nbuf = s.radices.size() >= 3 ? 2u : (s.radices.size() == 2 ? 1u : 0u);
 #else
-        // one buffer where no stage has more than one butterfly a thread
-        d.inplace = 1;
+        // one buffer where every stage is one round of butterflies, with more
+        // threads where that takes them (up to the limit of the plan)
+        uint32_t want_threads = kPassThreads;
         for (uint8_t r : s.radices)
-            if (!d.spec && uint64_t(C) * (s.R / r) > kPassThreads) d.inplace = 0;
+            want_threads = std::max<uint32_t>(want_threads, (C * (s.R / r) + fx_group(r) - 1) / fx_group(r));
+        want_threads = (want_threads + 31) / 32 * 32;
+        d.inplace = d.spec || want_threads <= std::min(kFxWideThreads, P.var.fx_threads) ? 1 : 0;
+        if (d.inplace) d.threads = want_threads;
         const uint32_t nbuf = d.inplace ? 1u : 2u;
-        d.fx = d.nrad > 0 && elems <= kFxElems * kPassThreads ? 1 : 0;
+        d.fx = d.nrad > 0 ? 1 : 0;
         if (d.spec) d.threads = std::max<uint32_t>(32, (elems / 8 + 31) / 32 * 32);
 #endif
         d.lane_stride = spec_lane_stride(s.R, C, d.load_mode == MODE_LANE,
@@ -651,6 +656,9 @@ static PassDesc make_desc(const FftPlan& P, size_t pi, const vec2_t* in, const L
 #if !defined(KFFT_HALF_SCALAR)
         d.fx_words = d.smem_bytes;
         d.smem_bytes += std::max<uint32_t>(d.nrad, kFxRows) * C * uint32_t(sizeof(uint32_t));
+        d.smem_bytes = (d.smem_bytes + 15u) & ~15u;
+        d.fx_lanes = d.smem_bytes;
+        if (!d.spec) d.smem_bytes += C * kFxLaneBytes;
 #endif
     } else {
         uint32_t t = (elems + 7) / 8;
@@ -671,6 +679,7 @@ static PassDesc make_desc(const FftPlan& P, size_t pi, const vec2_t* in, const L
     d.scale = scale;
 #if !defined(KFFT_HALF_SCALAR)
     d.fx_inner = s.fx_inner;
+    d.fx_one = 1;
     d.fx_lo = P.fx_lo;
     d.fx_hi = P.fx_hi;
     {

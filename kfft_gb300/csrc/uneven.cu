@@ -29,9 +29,10 @@ using namespace kfft;
 // KFFT_QUEUE_MINBLOCKS).  Tiles of at most 2048 points and passes of at most
 // 512, measured on the uneven batch of 3968 sequences: FP32 at four CTAs per
 // SM 9.38 ms against 9.96 ms for 4096 / 1024 at three (4096 / 512 at four:
-// 10.37 ms; 2048 / 512 at three: 11.48 ms; 1024 / 256 at four: 14.89 ms);
-// FP64 at three CTAs per SM 84.1 ms against 100.1 ms for 4096 / 1024 at two
-// (2048 / 512 at two: 87.7 ms).
+// 10.37 ms; 2048 / 512 at three: 11.48 ms; 1024 / 256 at four: 14.89 ms).
+// Double build (fixed-point tiles), 256 sequences of up to 2^18 points, as the
+// tiles stood: at two CTAs per SM 2048 / 512 1.12 ms, 2048 / 256 1.21 ms, 4096
+// / 512 1.77 ms; at three CTAs 2048 / 512 and 2048 / 1024 0.87 ms.
 #ifndef KFFT_QUEUE_TILE
 #define KFFT_QUEUE_TILE 2048
 #endif
@@ -329,6 +330,7 @@ KFFT_API kfft_plan_uneven* kfft_config_cpx_uneven(uint32_t count, const uint32_t
             if (var.no_fused) var = PlanVariant();
             var.tile_cap = std::min<uint32_t>(var.tile_cap, KFFT_QUEUE_TILE);
             var.rmax = std::min<uint32_t>(var.rmax, KFFT_QUEUE_RMAX);
+            var.fx_threads = KFFT_QUEUE_THREADS;
             FftPlan* fp = make_plan(n, sign, P->arena, st, kUnevenMaxPrime, var);
             if (!fp) return NULL;
             P->plans[n].reset(fp);

@@ -94,3 +94,25 @@ def test_ends_of_the_exponent_range(lib, n, e):
     # below 2^-1022 the inputs themselves lose bits
     lost = 2.0 ** (-1074 - e) * 4 if e < -1000 else 0.0
     assert rel_l2(got * 2.0 ** (-e // 2) * 2.0 ** (-e - (-e // 2)), ref) <= 1e-15 + lost
+
+
+def test_queue_tiles(lib):
+    """The queue kernel's tiles: every power of two it runs in one tile, and
+    lengths whose stages take one round of its threads or more."""
+    lengths = np.array([16, 32, 64, 128, 256, 512, 1024, 2048, 4096, 1 << 17, 11, 1792, 1820, 1848,
+                        1960, 2016, 2028, 2047, 1890, 1331, 2197, 30030, 4099, 65537, 9973], np.uint32)
+    rng = np.random.default_rng(3)
+    x = rng.standard_normal(int(lengths.sum())) + 1j * rng.standard_normal(int(lengths.sum()))
+    for flags, f in ((0, np.fft.fft), (K.FLAG_INVERSE, np.fft.ifft)):
+        p = lib.L.kfft_config_cpx_uneven(len(lengths), lengths.ctypes.data, flags)
+        assert p, lib.last_error()
+        y = np.empty_like(x)
+        r = lib.L.kfft_eval_cpx_uneven(p, x.ctypes.data, y.ctypes.data)
+        lib.L.kfft_release_uneven(p)
+        assert r == 0, lib.last_error()
+        at = 0
+        for n in lengths.tolist():
+            ref = f(x[at:at + n].astype(np.clongdouble))
+            # at most four passes a transform in the queue, and a convolution has three
+            assert float(np.linalg.norm(y[at:at + n] - ref) / np.linalg.norm(ref)) <= 14 * ULP, n
+            at += n
