@@ -1255,6 +1255,126 @@ __device__ __forceinline__ void tile_loop_pipelined(const PassDesc& d, vec2_t* s
 }
 
 #if defined(KFFT_HALF_SCALAR)
+// One middle radix-16 stage with its reads and writes in one buffer: one
+// butterfly a thread (C * R = 16 points a thread), a barrier between.
+template <uint32_t R, uint32_t NS, bool INV>
+__device__ __forceinline__ void spec_stage_inplace(const PassDesc& d, vec2_t* buf) {
+    constexpr uint32_t M = R / 16, TWS = R / (NS * 16);
+    // threads past the last butterfly repeat it without storing
+    const bool act = threadIdx.x < d.C * M;
+    const uint32_t it = act ? threadIdx.x : d.C * M - 1;
+    const uint32_t c = it / M, jj = it % M;
+    vec2_t* l0 = buf + c * d.lane_stride;
+    vec2_t v[16];
+#pragma unroll
+    for (int q = 0; q < 16; ++q) v[q] = l0[pad(jj + q * M)];
+    apply_inner_twiddles<16>(v, d.tw_inner, (jj % NS) * TWS);
+    dft<16, INV>(v);
+    const uint32_t ob = (jj / NS) * NS * 16 + jj % NS;
+    __syncthreads();
+    if (act) {
+#pragma unroll
+        for (int q = 0; q < 16; ++q) l0[pad(ob + q * NS)] = v[q];
+    }
+}
+
+// As tile_loop_pipelined, with the next tile's inputs on their way into
+// shared memory (cp.async) instead of registers, and one exchange buffer:
+// 80 registers and 66 KB a CTA, so three fit an SM (24 warps) where the
+// register-prefetching loop fits two.  These passes are bound by latency:
+// forward, us, two CTAs against three: 64 x 2^18 139 -> 129, 16 x 2^20 163 ->
+// 154, 2^24 175 -> 158 (5.1 TB/s a pass), and 1024-point passes beat 8192-point
+// tiles of 512 threads and one CTA (136 -> 129 for 64 x 2^18).
+// Shared memory: [raw tile, R rows of C lanes | exchange buffer].  Needs C * R
+// = 16 points a thread, lanes in rows (load mode LANE) and a plain prologue.
+// `pairs`: two neighbouring lanes lie 16-byte aligned side by side in every
+// row (one copy for both); otherwise each lane is copied by itself.
+template <uint32_t R, bool INV>
+__device__ __forceinline__ void tile_loop_async(const PassDesc& d, bool pairs, vec2_t* sm) {
+    constexpr uint32_t L = ilog2(R);
+    constexpr uint32_t K16 = L / 4;
+    constexpr int T = 1 << (L % 4);
+    constexpr int NP = int(K16) + (T > 1 ? 1 : 0);
+    constexpr int PL = T > 1 ? T : 16;
+    constexpr uint32_t M0 = R / 16;
+    const uint32_t total = d.batch * d.lanes_j;
+    const uint32_t lstride = d.lane_stride, C = d.C;
+    vec2_t* raw = sm;
+    vec2_t* buf = sm + C * R;
+    const uint32_t jj0 = threadIdx.x / C, c0 = threadIdx.x % C;  // C is a power of two
+    auto locate = [&](uint32_t g, uint32_t& bs, uint32_t& j) -> bool {
+        if (g >= total) return false;
+        if (d.order == ORDER_J) {
+            bs = fdiv(g, d.div_lanes_j);
+            j = g - bs * d.lanes_j;
+        } else {
+            j = fdiv(g, d.div_batch);
+            bs = g - j * d.batch;
+        }
+        return true;
+    };
+    // this thread's copies: lane cp (and the next one) of rows row0, row0 + rstep, ...
+    const uint32_t width = pairs ? 2u : 1u, per_row = C / width;
+    const uint32_t cp = width * (threadIdx.x % per_row), row0 = threadIdx.x / per_row;
+    const uint32_t rstep = blockDim.x / per_row;
+    const uint32_t raw_at = uint32_t(__cvta_generic_to_shared(raw + row0 * C + cp));
+    const uint32_t raw_step = rstep * C * uint32_t(sizeof(vec2_t));
+    auto issue = [&](uint32_t tile) {
+        uint32_t bs, j;
+        if (locate(tile * C + cp, bs, j)) {
+            const vec2_t* p = d.in + uint64_t(bs) * d.in_bs + uint64_t(j + row0 * d.lanes_j) * d.in_es;
+            const uint64_t step = uint64_t(rstep) * d.lanes_j * d.in_es;
+            if (pairs) {
+#pragma unroll
+                for (uint32_t i = 0; i < 8; ++i)
+                    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(raw_at + i * raw_step),
+                                 "l"(p + i * step)
+                                 : "memory");
+            } else {
+#pragma unroll
+                for (uint32_t i = 0; i < 16; ++i)
+                    asm volatile("cp.async.ca.shared.global [%0], [%1], 8;" ::"r"(raw_at + i * raw_step),
+                                 "l"(p + i * step)
+                                 : "memory");
+            }
+        }
+        asm volatile("cp.async.commit_group;" ::: "memory");
+    };
+    uint32_t tile = blockIdx.x;
+    if (tile < d.tiles) issue(tile);
+    for (; tile < d.tiles; tile += gridDim.x) {
+        asm volatile("cp.async.wait_group 0;" ::: "memory");
+        __syncthreads();
+        const uint32_t lane0 = tile * C;
+        vec2_t v[16];
+#pragma unroll
+        for (int q = 0; q < 16; ++q) v[q] = raw[(jj0 + q * M0) * C + c0];
+        __syncthreads();  // every read of raw is done: the next copies may land there
+        if (tile + gridDim.x < d.tiles) issue(tile + gridDim.x);
+        uint32_t bs = 0, j = 0;
+        const bool live = locate(lane0 + c0, bs, j);
+        if (live) outer_twiddle<16>(d, j, jj0, M0, v);
+        dft<16, INV>(v);
+        const uint32_t ob = jj0 * 16;
+        if constexpr (NP == 1) {
+            if (live) fused_store<16>(d, bs, j, ob, 1, v);
+        } else {
+            vec2_t* p0 = buf + c0 * lstride + pad(ob);  // 16 slots inside one pad period
+#pragma unroll
+            for (int q = 0; q < 16; ++q) p0[q] = v[q];
+            __syncthreads();
+            if constexpr (NP == 2) {
+                spec_stage<PL, R, 16, IO_SMEM, IO_GLOBAL, INV>(d, buf, nullptr, lane0, total);
+            } else {
+                spec_stage_inplace<R, 16, INV>(d, buf);
+                __syncthreads();
+                spec_stage<PL, R, 256, IO_SMEM, IO_GLOBAL, INV>(d, buf, nullptr, lane0, total);
+            }
+        }
+        // (the next tile's first barrier keeps its writes to buf behind these reads)
+    }
+}
+
 // ---------------------------------------------------------------------------
 // single-pass power-of-two tiles fed by one-dimensional bulk copies: the C
 // sequences of a tile are C*R contiguous points, so one untiled bulk copy
@@ -1307,7 +1427,7 @@ __device__ __forceinline__ bool mbar_wait(uint64_t* bar, uint32_t parity, uint32
     return false;
 }
 
-// Shared memory: [mbarrier | pad to 128 B | raw tile C*R | bufA | bufB].
+// Shared memory: [mbarrier | pad to 128 B | raw tile C*R | exchange buffer].
 // A wait that runs out after `max_polls` polls (only a failed or very slow
 // copy can cause it) sets *fail; the CTA then waits once more, with the
 // default limit, for the copy in flight to land and ends without finishing
@@ -1325,7 +1445,6 @@ __device__ __forceinline__ void tile_loop_bulk(const PassDesc& d, unsigned char*
     vec2_t* raw = reinterpret_cast<vec2_t*>(smem + 128);
     const uint32_t lstride = d.lane_stride;
     vec2_t* bufA = raw + d.C * R;
-    vec2_t* bufB = bufA + d.C * lstride + 1;
     const uint32_t total = d.batch;  // one lane per sequence (lanes_j == 1)
     const uint32_t it = threadIdx.x;
     const bool act = it < d.C * M0;
@@ -1389,9 +1508,9 @@ __device__ __forceinline__ void tile_loop_bulk(const PassDesc& d, unsigned char*
             spec_stage<PL, R, 16, IO_SMEM, IO_GLOBAL, INV>(d, bufA, nullptr, lane0, total);
         } else if constexpr (NP == 3) {
             __syncthreads();
-            spec_stage<16, R, 16, IO_SMEM, IO_SMEM, INV>(d, bufA, bufB, lane0, total);
+            spec_stage_inplace<R, 16, INV>(d, bufA);
             __syncthreads();
-            spec_stage<PL, R, 256, IO_SMEM, IO_GLOBAL, INV>(d, bufB, nullptr, lane0, total);
+            spec_stage<PL, R, 256, IO_SMEM, IO_GLOBAL, INV>(d, bufA, nullptr, lane0, total);
         }
         __syncthreads();  // the next tile's first stage overwrites bufA
     }

@@ -20,25 +20,16 @@ __global__ void __launch_bounds__(kPassThreads, KFFT_REG_MINBLOCKS) k_pass_reg(c
 
 // FP32 power-of-two passes, one kernel per pass length R so each kernel holds
 // only its own body (a small instruction footprint):
-// * k_pass_pipe: a plain prologue and more tiles than fit the GPU at once: a
-//   grid of resident CTAs, each running many tiles with its next tile's loads
-//   in flight (tile_loop_pipelined);
+// * k_pass_async: a plain prologue, full tiles of lanes in rows and more tiles
+//   than fit the GPU at once: a grid of resident CTAs, each running many tiles
+//   with its next tile on its way into shared memory (tile_loop_async);
+// * k_pass_pipe: the same for other tiles, the next tile's loads in registers
+//   (tile_loop_pipelined);
 // * k_pass_spec: one tile per CTA otherwise.
 // The FP64 build uses neither: the FP64 pipe, not index arithmetic or load
 // latency, bounds that path, and its unrolled bodies would spill.
 template <uint32_t R, bool INV>
 __global__ void __launch_bounds__(kPassThreads, 2) k_pass_pipe(const __grid_constant__ PassDesc d) {
-    extern __shared__ __align__(16) unsigned char smem_raw[];
-    tile_loop_pipelined<R, INV>(d, reinterpret_cast<vec2_t*>(smem_raw));
-}
-
-// k_pass_pipe with twice the threads and twice the lanes per tile (8192
-// points): multi-lane passes of 512 or 1024 points, whose 4096-point tiles
-// hold only 8 or 4 lanes (64- or 32-byte row segments), read and write twice
-// as wide segments.  One CTA per SM.  (256-point passes, whose 4096-point
-// tiles already hold 16 lanes, measured slower on it.)
-template <uint32_t R, bool INV>
-__global__ void __launch_bounds__(2 * kPassThreads, 1) k_pass_pipe_wide(const __grid_constant__ PassDesc d) {
     extern __shared__ __align__(16) unsigned char smem_raw[];
     tile_loop_pipelined<R, INV>(d, reinterpret_cast<vec2_t*>(smem_raw));
 }
@@ -51,6 +42,13 @@ __global__ void __launch_bounds__(kPassThreads, KFFT_REG_MINBLOCKS) k_pass_spec(
     tile_body_spec<R, INV>(d, blockIdx.x * d.C, d.batch * d.lanes_j, sm, sm + d.C * d.lane_stride + 1);
 }
 
+template <uint32_t R, bool INV>
+__global__ void __launch_bounds__(kPassThreads, 3) k_pass_async(const __grid_constant__ PassDesc d,
+                                                                uint32_t pairs) {
+    extern __shared__ __align__(16) unsigned char smem_raw[];
+    tile_loop_async<R, INV>(d, pairs != 0, reinterpret_cast<vec2_t*>(smem_raw));
+}
+
 // Set when a bulk-copy wait of k_pass_bulk ran out (only a failed or very
 // slow copy can cause it); the CTA then ends without finishing its tiles.
 // One word per host-thread slot: a launch passes its thread's slot, and the
@@ -59,9 +57,11 @@ __global__ void __launch_bounds__(kPassThreads, KFFT_REG_MINBLOCKS) k_pass_spec(
 __device__ uint32_t g_bulk_wait_failed[kWaitSlots];
 
 // Single-pass FP32 power-of-two batches of contiguous sequences: each tile's
-// points arrive by one bulk copy (tile_loop_bulk).
+// points arrive by one bulk copy (tile_loop_bulk).  One exchange buffer and 80
+// registers, so three CTAs an SM: 4096 x 4096 points forward 63.6 us, 66 with
+// two buffers and two CTAs (2048-point sequences 65.7 -> 60.5).
 template <uint32_t R, bool INV>
-__global__ void __launch_bounds__(kPassThreads, 2) k_pass_bulk(const __grid_constant__ PassDesc d,
+__global__ void __launch_bounds__(kPassThreads, 3) k_pass_bulk(const __grid_constant__ PassDesc d,
                                                                uint32_t slot, uint32_t max_polls) {
     extern __shared__ __align__(128) unsigned char smem_raw[];
     tile_loop_bulk<R, INV>(d, smem_raw, &g_bulk_wait_failed[slot], max_polls);
@@ -70,22 +70,32 @@ __global__ void __launch_bounds__(kPassThreads, 2) k_pass_bulk(const __grid_cons
 using SpecKernel = void (*)(PassDesc);
 using BulkKernel = void (*)(PassDesc, uint32_t, uint32_t);
 
-// shortest pass that runs on the wide tiles
-#ifndef KFFT_WIDE_MIN_R
-#define KFFT_WIDE_MIN_R 512
-#endif
+using AsyncKernel = void (*)(PassDesc, uint32_t);
 
-enum SpecKind { SPEC_ONE_TILE = 0, SPEC_PIPE = 1, SPEC_WIDE = 3 };
+enum SpecKind { SPEC_ONE_TILE = 0, SPEC_PIPE = 1 };
 
 template <uint32_t R>
 SpecKernel pick(int kind, bool inv) {
-    if constexpr (R >= 256 && R <= 1024) {
-        if (kind == SPEC_WIDE) return inv ? k_pass_pipe_wide<R, true> : k_pass_pipe_wide<R, false>;
-    } else {
-        if (kind == SPEC_WIDE) return nullptr;
-    }
     if (kind == SPEC_PIPE) return inv ? k_pass_pipe<R, true> : k_pass_pipe<R, false>;
     return inv ? k_pass_spec<R, true> : k_pass_spec<R, false>;
+}
+
+template <uint32_t R>
+AsyncKernel pick_async(bool inv) {
+    return inv ? k_pass_async<R, true> : k_pass_async<R, false>;
+}
+
+AsyncKernel async_kernel(uint32_t spec, bool inv) {
+    switch (spec) {
+        case 4: return pick_async<16>(inv);
+        case 5: return pick_async<32>(inv);
+        case 6: return pick_async<64>(inv);
+        case 7: return pick_async<128>(inv);
+        case 8: return pick_async<256>(inv);
+        case 9: return pick_async<512>(inv);
+        case 10: return pick_async<1024>(inv);
+        default: return nullptr;
+    }
 }
 
 template <uint32_t R>
@@ -226,7 +236,7 @@ void launch_pass_reg(const PassDesc& d, const PassExtra& x, cudaStream_t st) {
                                 d.in_bs == d.R && (reinterpret_cast<uintptr_t>(d.in) & 15u) == 0;
         if (d.pro_op == PRO_NONE && contiguous) {
             BulkKernel f = bulk_kernel(d.spec, inv);
-            const uint32_t smem = 128 + d.C * d.R * uint32_t(sizeof(vec2_t)) + d.smem_bytes;
+            const uint32_t smem = 128 + (d.C * d.R + d.C * d.lane_stride + 1u) * uint32_t(sizeof(vec2_t));
             const int per_sm = f ? prepare((const void*)f, smem) : -1;
             const uint32_t grid = uint32_t(std::max(per_sm, 0)) * uint32_t(sm_count());
             if (per_sm > 0 && d.tiles >= 2 * grid) {
@@ -237,24 +247,21 @@ void launch_pass_reg(const PassDesc& d, const PassExtra& x, cudaStream_t st) {
                 return;
             }
         }
-        // multi-lane rows of 256-1024 points with a full 4096-point tile:
-        // the same pass on 8192-point tiles of twice the lanes
-        if (d.pro_op == PRO_NONE && d.order == ORDER_J && d.R >= KFFT_WIDE_MIN_R && d.R <= 1024 &&
-            d.C * d.R == kRegTile && d.lanes_j >= 2 * d.C) {
-            SpecKernel f = spec_kernel(d.spec, SPEC_WIDE, inv);
-            PassDesc w = d;
-            w.C = 2 * d.C;
-            w.div_C.init(w.C);
-            w.tiles = uint32_t((uint64_t(d.batch) * d.lanes_j + w.C - 1) / w.C);
-            w.threads = 2 * kPassThreads;
-            w.lane_stride = spec_lane_stride(d.R, w.C, d.load_mode == MODE_LANE,
-                                             d.store_mode == MODE_LANE, w.threads);
-            const uint32_t nbuf = d.R == 256 ? 1u : 2u;  // stages 16,16 or 16,16,T
-            w.smem_bytes = nbuf * (w.C * w.lane_stride + 1u) * uint32_t(sizeof(vec2_t));
-            const int per_sm = f ? prepare((const void*)f, w.smem_bytes, w.threads) : -1;
+        // full tiles of lanes in rows (passes of up to 1024 points, so at
+        // least four lanes): copied asynchronously, two lanes at a time where
+        // they lie together on 16 bytes in every row
+        if (d.pro_op == PRO_NONE && d.load_mode == MODE_LANE && d.C * d.R == kRegTile && d.C >= 4) {
+            const bool rows_even = d.order == ORDER_J
+                                       ? d.in_es == 1 && d.lanes_j % 2 == 0 && d.in_bs % 2 == 0
+                                       : d.in_bs == 1 && d.in_es % 2 == 0 && d.batch % 2 == 0;
+            const bool pairs = rows_even && (reinterpret_cast<uintptr_t>(d.in) & 15u) == 0;
+            AsyncKernel f = async_kernel(d.spec, inv);
+            const uint32_t smem =
+                (d.C * d.R + d.C * d.lane_stride + 1u) * uint32_t(sizeof(vec2_t));
+            const int per_sm = f ? prepare((const void*)f, smem) : -1;
             const uint32_t grid = uint32_t(std::max(per_sm, 0)) * uint32_t(sm_count());
-            if (per_sm > 0 && w.tiles >= 2 * grid) {
-                f<<<grid, w.threads, w.smem_bytes, st>>>(w);
+            if (per_sm > 0 && d.tiles >= 2 * grid) {
+                f<<<grid, kPassThreads, smem, st>>>(d, pairs ? 1u : 0u);
                 note_cuda_error(cudaGetLastError());
                 count_launch();
                 return;

@@ -319,10 +319,12 @@ inline uint32_t lane_stride_search(uint32_t R, uint32_t C, bool load_lane, bool 
 // most 1024), longest first, with the least estimated time.  A pass costs its
 // measured launch time relative to a 256-point pass on 2^24 points: up to 256
 // points 1 (tiles of 16+ lanes, row segments of 128 bytes or more), 512
-// points 1.44 and 1024 points 1.65 (8 and 4 lanes per 4096-point tile, 16 and
-// 8 on the wide kernel).  Ties go to fewer passes, then to the more even
-// split (lexicographically smaller lengths, longest first).  2^18 runs as 1024 x 256 (0.292 ms per forward + inverse
-// step at 64 sequences, against 0.315 as 512 x 512), 2^20 as 128 x 128 x 64.
+// points 1.44 and 1024 points 1.65 (8 and 4 lanes per 4096-point tile; 1.35
+// and 1.5 with k_pass_async, which leaves the choices as they are).  Ties go to
+// fewer passes, then to the more even split (lexicographically smaller lengths,
+// longest first).  Forward, us: 64 x 2^18 as 1024 x 256 128 (512 x 512 141, 64 x
+// 64 x 64 154), 16 x 2^20 as 128 x 128 x 64 153 (1024 x 1024 165), 2^24 as 256 x
+// 256 x 256 157 (4096 x 4096, one lane a tile, 692).
 inline std::vector<uint32_t> pow2_split(uint32_t N, uint32_t rmax) {
     uint32_t L = 0;
     while ((1u << L) < N) ++L;
