@@ -29,6 +29,8 @@ SOURCES = ["pass_smem.cu", "pass_reg.cu", "persistent.cu", "tables.cu", "plan.cu
 # device code across objects (-rdc), the FP64 tile within 64 registers.
 FX_SOURCES = [("fp64_tile.cu", "fp64_tile", ["-maxrregcount=64"])]
 FX_SOURCES += [("pass_fx.cu", f"pass_fx{p}", [f"-DKFFT_FX_PART={p}"]) for p in range(4)]
+# Float build only: the parts of the register-tile kernels.
+REG_SOURCES = [("pass_reg.cu", f"pass_reg{p}", [f"-DKFFT_REG_PART={p}"]) for p in (1, 2, 3)]
 RDC = {"persistent.cu", "fp64_tile.cu", "pass_fx.cu"}
 HEADERS = ["engine.cuh", "fft_device.cuh", "fx_math.cuh", "fx_spec.cuh", "fx_tile.cuh", "plan_host.h"]
 ARCH = ["-gencode", "arch=compute_103a,code=sm_103a"]
@@ -72,7 +74,7 @@ def build(force: bool = False, verbose: bool = False) -> dict[str, str]:
             continue
         tag = lib.replace(".so", "")
         objs = []
-        units = [(s, s[:-3], []) for s in SOURCES] + ([] if defines else FX_SOURCES)
+        units = [(s, s[:-3], []) for s in SOURCES] + (REG_SOURCES if defines else FX_SOURCES)
         for s, name, more in units:
             obj = os.path.join(OBJ_DIR, f"{tag}_{name}.o")
             objs.append(obj)

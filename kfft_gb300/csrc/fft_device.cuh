@@ -746,19 +746,73 @@ __device__ __forceinline__ void fused_load(const PassDesc& d, uint32_t bs, uint3
     outer_twiddle<P>(d, j, jj, m, v);
 }
 
+// Which epilogues a kernel is compiled for: any (one element after the other),
+// the plain store only, or the others with a product's factors loaded four at
+// a time before the stores.  (All in one kernel cost the plain store: 4096 x
+// 4096 points 73.7 us against 63.6.  In kernels that switch between many
+// bodies at run time the grouped code is shared between them and spilled
+// around, so those keep the first form.)
+enum : int { STORE_ANY = 0, STORE_PLAIN = 1, STORE_PRODUCT = 2 };
+
 // Stores the P outputs of one butterfly of the last inner pass straight to
 // global memory through the epilogue.
-template <int P>
+template <int P, int STORE = STORE_ANY>
 __device__ __forceinline__ void fused_store(const PassDesc& d, uint32_t bs, uint32_t j, uint32_t ob,
                                             uint32_t ns, const vec2_t* v) {
     const uint32_t blo = fdiv(j, d.div_Ns);
     const uint32_t ko = j - blo * d.Ns;
     const uint32_t base = blo * d.Ns * d.R + ko;
-    if (d.epi_op == EPI_NONE) {
+    if (STORE == STORE_PLAIN || (STORE == STORE_ANY && d.epi_op == EPI_NONE)) {
         vec2_t* o = d.out + uint64_t(bs) * d.out_bs;
         const uint64_t es = d.out_es;
 #pragma unroll
         for (int q = 0; q < P; ++q) o[uint64_t(base + (ob + q * ns) * d.Ns) * es] = cscale(v[q], d.scale);
+    } else if (STORE == STORE_PRODUCT && d.epi_op == EPI_RADER_INV) {
+        constexpr int G = P < 8 ? P : 8;
+        const uint32_t k = base + ob * d.Ns, ks = ns * d.Ns;
+        vec2_t* o = d.aux_out + uint64_t(bs) * d.aux_out_bs;
+        if (k == 0) o[0] = cscale(__ldcg(&d.aux_in[bs]), d.scale);
+#pragma unroll
+        for (int g = 0; g < P; g += G) {
+            uint32_t at[G];
+#pragma unroll
+            for (int u = 0; u < G; ++u)
+                if (g + u < P) at[u] = __ldg(&d.epi_perm[k + (g + u) * ks]);
+#pragma unroll
+            for (int u = 0; u < G; ++u)
+                if (g + u < P) o[uint64_t(at[u]) * d.aux_out_es] = cscale(v[g + u], d.scale);
+        }
+    } else if (STORE == STORE_PRODUCT) {
+        // (loading and storing one after the other took twice the time: 34 x
+        // 2^20 points, 64-point pass, 203 us against 95 without a product)
+        constexpr int G = P < 4 ? P : 4;
+        const bool own_layout = d.epi_op == EPI_MUL_OUT;
+        uint32_t k = base + ob * d.Ns;
+        const uint32_t ks = ns * d.Ns, bound = d.epi_op == EPI_CHIRP ? d.epi_bound : 0xffffffffu;
+        const uint64_t es = d.out_es, ts = own_layout ? es : 1;
+        vec2_t* o = d.out + uint64_t(bs) * d.out_bs;
+        const vec2_t* t = own_layout ? d.epi_tab + uint64_t(bs) * d.out_bs : d.epi_tab;
+        const real_t scale = own_layout || d.epi_op == EPI_CHIRP ? d.scale : real_t(1);
+        const bool rader = d.epi_op == EPI_RADER_FWD;
+#pragma unroll
+        for (int g = 0; g < P; g += G) {
+            vec2_t w[G];
+#pragma unroll
+            for (int u = 0; u < G; ++u)
+                if (g + u < P && k + u * ks < bound) w[u] = __ldcg(&t[uint64_t(k + u * ks) * ts]);
+#pragma unroll
+            for (int u = 0; u < G; ++u)
+                if (g + u < P && k + u * ks < bound) {
+                    vec2_t r = cscale(cmul(v[g + u], w[u]), scale);
+                    if (g + u == 0 && rader && k == 0) {  // (as in store_elem)
+                        const vec2_t x0 = __ldcg(&d.aux_in[uint64_t(bs) * d.aux_in_bs]);
+                        d.aux_out[bs] = cadd(x0, v[0]);
+                        r = cadd(r, x0);
+                    }
+                    o[uint64_t(k + u * ks) * es] = r;
+                }
+            k += G * ks;
+        }
     } else {
 #pragma unroll
         for (int q = 0; q < P; ++q) store_elem(d, bs, base + (ob + q * ns) * d.Ns, v[q]);
@@ -1053,7 +1107,7 @@ __device__ __forceinline__ void tc_pass16(const PassDesc& d, const InnerStep& st
 // multiple of the pad period, or a unit stride inside one period) they are
 // one base plus immediate offsets.
 // ---------------------------------------------------------------------------
-template <int P, uint32_t R, uint32_t NS, int SIO, int DIO, bool INV>
+template <int P, uint32_t R, uint32_t NS, int SIO, int DIO, bool INV, int STORE = STORE_ANY>
 __device__ __forceinline__ void spec_stage(const PassDesc& d, const vec2_t* __restrict__ src,
                                            vec2_t* __restrict__ dst, uint32_t lane0,
                                            uint32_t total) {
@@ -1122,7 +1176,7 @@ __device__ __forceinline__ void spec_stage(const PassDesc& d, const vec2_t* __re
                 for (int q = 0; q < P; ++q) l0[pad(ob + q * NS)] = v[q];
             }
         } else if (live) {
-            fused_store<P>(d, bs, j, ob, NS, v);
+            fused_store<P, STORE>(d, bs, j, ob, NS, v);
         }
     }
 }
@@ -1289,7 +1343,7 @@ __device__ __forceinline__ void spec_stage_inplace(const PassDesc& d, vec2_t* bu
 // = 16 points a thread, lanes in rows (load mode LANE) and a plain prologue.
 // `pairs`: two neighbouring lanes lie 16-byte aligned side by side in every
 // row (one copy for both); otherwise each lane is copied by itself.
-template <uint32_t R, bool INV>
+template <uint32_t R, bool INV, int STORE>
 __device__ __forceinline__ void tile_loop_async(const PassDesc& d, bool pairs, vec2_t* sm) {
     constexpr uint32_t L = ilog2(R);
     constexpr uint32_t K16 = L / 4;
@@ -1357,18 +1411,18 @@ __device__ __forceinline__ void tile_loop_async(const PassDesc& d, bool pairs, v
         dft<16, INV>(v);
         const uint32_t ob = jj0 * 16;
         if constexpr (NP == 1) {
-            if (live) fused_store<16>(d, bs, j, ob, 1, v);
+            if (live) fused_store<16, STORE>(d, bs, j, ob, 1, v);
         } else {
             vec2_t* p0 = buf + c0 * lstride + pad(ob);  // 16 slots inside one pad period
 #pragma unroll
             for (int q = 0; q < 16; ++q) p0[q] = v[q];
             __syncthreads();
             if constexpr (NP == 2) {
-                spec_stage<PL, R, 16, IO_SMEM, IO_GLOBAL, INV>(d, buf, nullptr, lane0, total);
+                spec_stage<PL, R, 16, IO_SMEM, IO_GLOBAL, INV, STORE>(d, buf, nullptr, lane0, total);
             } else {
                 spec_stage_inplace<R, 16, INV>(d, buf);
                 __syncthreads();
-                spec_stage<PL, R, 256, IO_SMEM, IO_GLOBAL, INV>(d, buf, nullptr, lane0, total);
+                spec_stage<PL, R, 256, IO_SMEM, IO_GLOBAL, INV, STORE>(d, buf, nullptr, lane0, total);
             }
         }
         // (the next tile's first barrier keeps its writes to buf behind these reads)
@@ -1432,7 +1486,7 @@ __device__ __forceinline__ bool mbar_wait(uint64_t* bar, uint32_t parity, uint32
 // copy can cause it) sets *fail; the CTA then waits once more, with the
 // default limit, for the copy in flight to land and ends without finishing
 // its tiles, so the caller must treat the output as invalid.
-template <uint32_t R, bool INV>
+template <uint32_t R, bool INV, int STORE>
 __device__ __forceinline__ void tile_loop_bulk(const PassDesc& d, unsigned char* smem,
                                                uint32_t* fail, uint32_t max_polls) {
     constexpr uint32_t L = ilog2(R);
@@ -1496,7 +1550,7 @@ __device__ __forceinline__ void tile_loop_bulk(const PassDesc& d, unsigned char*
             dft<16, INV>(v);
             const uint32_t ob = jj0 * 16;
             if constexpr (NP == 1) {
-                if (live) fused_store<16>(d, g, 0, ob, 1, v);
+                if (live) fused_store<16, STORE>(d, g, 0, ob, 1, v);
             } else {
                 vec2_t* p0 = bufA + c0 * lstride + pad(ob);  // 16 slots inside one pad period
 #pragma unroll
@@ -1505,12 +1559,12 @@ __device__ __forceinline__ void tile_loop_bulk(const PassDesc& d, unsigned char*
         }
         if constexpr (NP == 2) {
             __syncthreads();
-            spec_stage<PL, R, 16, IO_SMEM, IO_GLOBAL, INV>(d, bufA, nullptr, lane0, total);
+            spec_stage<PL, R, 16, IO_SMEM, IO_GLOBAL, INV, STORE>(d, bufA, nullptr, lane0, total);
         } else if constexpr (NP == 3) {
             __syncthreads();
             spec_stage_inplace<R, 16, INV>(d, bufA);
             __syncthreads();
-            spec_stage<PL, R, 256, IO_SMEM, IO_GLOBAL, INV>(d, bufA, nullptr, lane0, total);
+            spec_stage<PL, R, 256, IO_SMEM, IO_GLOBAL, INV, STORE>(d, bufA, nullptr, lane0, total);
         }
         __syncthreads();  // the next tile's first stage overwrites bufA
     }

@@ -1,4 +1,6 @@
-// pass_reg.cu -- the register-resident pass kernel k_pass_reg.
+// pass_reg.cu -- the register-resident pass kernels of the FP32 build: the
+// generic k_pass_reg, the compile-time power-of-two kernels and their
+// launcher.  Built in parts (KFFT_REG_PART) that compile in parallel.
 #include "fft_device.cuh"
 
 #include <algorithm>
@@ -7,16 +9,23 @@
 #include <mutex>
 #include <utility>
 
+#ifndef KFFT_REG_PART
+#define KFFT_REG_PART 0
+#endif
+
 namespace kfft {
 
 #if defined(KFFT_HALF_SCALAR)
-template <bool INV>
-__global__ void __launch_bounds__(kPassThreads, KFFT_REG_MINBLOCKS) k_pass_reg(const __grid_constant__ PassDesc d,
-                                                              const __grid_constant__ PassExtra x) {
-    extern __shared__ __align__(16) unsigned char smem_raw[];
-    // power-of-two FP32 passes launch k_pass_spec / k_pass_pipe instead
-    tile_body_reg<INV, false>(d, x, blockIdx.x, reinterpret_cast<vec2_t*>(smem_raw));
-}
+using SpecKernel = void (*)(PassDesc);
+using AsyncKernel = void (*)(PassDesc, uint32_t);
+using BulkKernel = void (*)(PassDesc, uint32_t*, uint32_t);
+
+enum SpecKind { SPEC_ONE_TILE = 0, SPEC_PIPE = 1 };
+
+// the kernels of a pass of 2^spec points (null: none)
+SpecKernel spec_kernel(uint32_t spec, int kind, bool inv);
+AsyncKernel async_kernel(uint32_t spec, bool inv, bool plain);
+BulkKernel bulk_kernel(uint32_t spec, bool inv, bool plain);
 
 // FP32 power-of-two passes, one kernel per pass length R so each kernel holds
 // only its own body (a small instruction footprint):
@@ -26,8 +35,7 @@ __global__ void __launch_bounds__(kPassThreads, KFFT_REG_MINBLOCKS) k_pass_reg(c
 // * k_pass_pipe: the same for other tiles, the next tile's loads in registers
 //   (tile_loop_pipelined);
 // * k_pass_spec: one tile per CTA otherwise.
-// The FP64 build uses neither: the FP64 pipe, not index arithmetic or load
-// latency, bounds that path, and its unrolled bodies would spill.
+#if KFFT_REG_PART == 1
 template <uint32_t R, bool INV>
 __global__ void __launch_bounds__(kPassThreads, 2) k_pass_pipe(const __grid_constant__ PassDesc d) {
     extern __shared__ __align__(16) unsigned char smem_raw[];
@@ -42,80 +50,10 @@ __global__ void __launch_bounds__(kPassThreads, KFFT_REG_MINBLOCKS) k_pass_spec(
     tile_body_spec<R, INV>(d, blockIdx.x * d.C, d.batch * d.lanes_j, sm, sm + d.C * d.lane_stride + 1);
 }
 
-template <uint32_t R, bool INV>
-__global__ void __launch_bounds__(kPassThreads, 3) k_pass_async(const __grid_constant__ PassDesc d,
-                                                                uint32_t pairs) {
-    extern __shared__ __align__(16) unsigned char smem_raw[];
-    tile_loop_async<R, INV>(d, pairs != 0, reinterpret_cast<vec2_t*>(smem_raw));
-}
-
-// Set when a bulk-copy wait of k_pass_bulk ran out (only a failed or very
-// slow copy can cause it); the CTA then ends without finishing its tiles.
-// One word per host-thread slot: a launch passes its thread's slot, and the
-// thread's next synchronous completion (take_wait_failures) reads and clears
-// it, so the failure becomes that call's return code.
-__device__ uint32_t g_bulk_wait_failed[kWaitSlots];
-
-// Single-pass FP32 power-of-two batches of contiguous sequences: each tile's
-// points arrive by one bulk copy (tile_loop_bulk).  One exchange buffer and 80
-// registers, so three CTAs an SM: 4096 x 4096 points forward 63.6 us, 66 with
-// two buffers and two CTAs (2048-point sequences 65.7 -> 60.5).
-template <uint32_t R, bool INV>
-__global__ void __launch_bounds__(kPassThreads, 3) k_pass_bulk(const __grid_constant__ PassDesc d,
-                                                               uint32_t slot, uint32_t max_polls) {
-    extern __shared__ __align__(128) unsigned char smem_raw[];
-    tile_loop_bulk<R, INV>(d, smem_raw, &g_bulk_wait_failed[slot], max_polls);
-}
-
-using SpecKernel = void (*)(PassDesc);
-using BulkKernel = void (*)(PassDesc, uint32_t, uint32_t);
-
-using AsyncKernel = void (*)(PassDesc, uint32_t);
-
-enum SpecKind { SPEC_ONE_TILE = 0, SPEC_PIPE = 1 };
-
 template <uint32_t R>
 SpecKernel pick(int kind, bool inv) {
     if (kind == SPEC_PIPE) return inv ? k_pass_pipe<R, true> : k_pass_pipe<R, false>;
     return inv ? k_pass_spec<R, true> : k_pass_spec<R, false>;
-}
-
-template <uint32_t R>
-AsyncKernel pick_async(bool inv) {
-    return inv ? k_pass_async<R, true> : k_pass_async<R, false>;
-}
-
-AsyncKernel async_kernel(uint32_t spec, bool inv) {
-    switch (spec) {
-        case 4: return pick_async<16>(inv);
-        case 5: return pick_async<32>(inv);
-        case 6: return pick_async<64>(inv);
-        case 7: return pick_async<128>(inv);
-        case 8: return pick_async<256>(inv);
-        case 9: return pick_async<512>(inv);
-        case 10: return pick_async<1024>(inv);
-        default: return nullptr;
-    }
-}
-
-template <uint32_t R>
-BulkKernel pick_bulk(bool inv) {
-    return inv ? k_pass_bulk<R, true> : k_pass_bulk<R, false>;
-}
-
-BulkKernel bulk_kernel(uint32_t spec, bool inv) {
-    switch (spec) {
-        case 4: return pick_bulk<16>(inv);
-        case 5: return pick_bulk<32>(inv);
-        case 6: return pick_bulk<64>(inv);
-        case 7: return pick_bulk<128>(inv);
-        case 8: return pick_bulk<256>(inv);
-        case 9: return pick_bulk<512>(inv);
-        case 10: return pick_bulk<1024>(inv);
-        case 11: return pick_bulk<2048>(inv);
-        case 12: return pick_bulk<4096>(inv);
-        default: return nullptr;
-    }
 }
 
 SpecKernel spec_kernel(uint32_t spec, int kind, bool inv) {
@@ -134,12 +72,106 @@ SpecKernel spec_kernel(uint32_t spec, int kind, bool inv) {
 }
 #endif
 
+#if KFFT_REG_PART == 2
+template <uint32_t R, bool INV, int STORE>
+__global__ void __launch_bounds__(kPassThreads, 3) k_pass_async(const __grid_constant__ PassDesc d,
+                                                                uint32_t pairs) {
+    extern __shared__ __align__(16) unsigned char smem_raw[];
+    tile_loop_async<R, INV, STORE>(d, pairs != 0, reinterpret_cast<vec2_t*>(smem_raw));
+}
+
+template <uint32_t R>
+AsyncKernel pick_async(bool inv, bool plain) {
+    if (plain) return inv ? k_pass_async<R, true, STORE_PLAIN> : k_pass_async<R, false, STORE_PLAIN>;
+    return inv ? k_pass_async<R, true, STORE_PRODUCT> : k_pass_async<R, false, STORE_PRODUCT>;
+}
+
+AsyncKernel async_kernel(uint32_t spec, bool inv, bool plain) {
+    switch (spec) {
+        case 4: return pick_async<16>(inv, plain);
+        case 5: return pick_async<32>(inv, plain);
+        case 6: return pick_async<64>(inv, plain);
+        case 7: return pick_async<128>(inv, plain);
+        case 8: return pick_async<256>(inv, plain);
+        case 9: return pick_async<512>(inv, plain);
+        case 10: return pick_async<1024>(inv, plain);
+        default: return nullptr;
+    }
+}
+#endif
+
+#if KFFT_REG_PART == 3
+// Single-pass FP32 power-of-two batches of contiguous sequences: each tile's
+// points arrive by one bulk copy (tile_loop_bulk).  One exchange buffer and 80
+// registers, so three CTAs an SM: 4096 x 4096 points forward 63.6 us, 66 with
+// two buffers and two CTAs (2048-point sequences 65.7 -> 60.5).
+// `fail` is set when a copy's wait runs out (g_bulk_wait_failed).
+template <uint32_t R, bool INV, int STORE>
+__global__ void __launch_bounds__(kPassThreads, 3) k_pass_bulk(const __grid_constant__ PassDesc d,
+                                                               uint32_t* fail, uint32_t max_polls) {
+    extern __shared__ __align__(128) unsigned char smem_raw[];
+    tile_loop_bulk<R, INV, STORE>(d, smem_raw, fail, max_polls);
+}
+
+template <uint32_t R>
+BulkKernel pick_bulk(bool inv, bool plain) {
+    if (plain) return inv ? k_pass_bulk<R, true, STORE_PLAIN> : k_pass_bulk<R, false, STORE_PLAIN>;
+    return inv ? k_pass_bulk<R, true, STORE_PRODUCT> : k_pass_bulk<R, false, STORE_PRODUCT>;
+}
+
+BulkKernel bulk_kernel(uint32_t spec, bool inv, bool plain) {
+    switch (spec) {
+        case 4: return pick_bulk<16>(inv, plain);
+        case 5: return pick_bulk<32>(inv, plain);
+        case 6: return pick_bulk<64>(inv, plain);
+        case 7: return pick_bulk<128>(inv, plain);
+        case 8: return pick_bulk<256>(inv, plain);
+        case 9: return pick_bulk<512>(inv, plain);
+        case 10: return pick_bulk<1024>(inv, plain);
+        case 11: return pick_bulk<2048>(inv, plain);
+        case 12: return pick_bulk<4096>(inv, plain);
+        default: return nullptr;
+    }
+}
+#endif
+#endif
+
+#if KFFT_REG_PART == 0
+#if defined(KFFT_HALF_SCALAR)
+template <bool INV>
+__global__ void __launch_bounds__(kPassThreads, KFFT_REG_MINBLOCKS) k_pass_reg(const __grid_constant__ PassDesc d,
+                                                              const __grid_constant__ PassExtra x) {
+    extern __shared__ __align__(16) unsigned char smem_raw[];
+    // power-of-two FP32 passes launch k_pass_spec / k_pass_pipe instead
+    tile_body_reg<INV, false>(d, x, blockIdx.x, reinterpret_cast<vec2_t*>(smem_raw));
+}
+
+// Set when a bulk-copy wait of k_pass_bulk ran out (only a failed or very
+// slow copy can cause it); the CTA then ends without finishing its tiles.
+// One word per host-thread slot: a launch passes its thread's slot, and the
+// thread's next synchronous completion (take_wait_failures) reads and clears
+// it, so the failure becomes that call's return code.
+__device__ uint32_t g_bulk_wait_failed[kWaitSlots];
+#endif
+
 namespace {
 std::atomic<uint32_t> g_bulk_polls{kBulkMaxPolls};
 std::atomic<int> g_slot_next{0};
 thread_local bool t_bulk_launched = false;
 
 #if defined(KFFT_HALF_SCALAR)
+// device address of the failure flags (null: the lookup failed)
+uint32_t* wait_flags() {
+    static uint32_t* const p = [] {
+        void* v = nullptr;
+        if (cudaGetSymbolAddress(&v, g_bulk_wait_failed) != cudaSuccess) {
+            cudaGetLastError();
+            v = nullptr;
+        }
+        return static_cast<uint32_t*>(v);
+    }();
+    return p;
+}
 uint32_t bulk_wait_polls() { return g_bulk_polls.load(std::memory_order_relaxed); }
 void note_bulk_launch() { t_bulk_launched = true; }
 
@@ -235,12 +267,13 @@ void launch_pass_reg(const PassDesc& d, const PassExtra& x, cudaStream_t st) {
         const bool contiguous = d.lanes_j == 1 && d.order == ORDER_J && d.in_es == 1 &&
                                 d.in_bs == d.R && (reinterpret_cast<uintptr_t>(d.in) & 15u) == 0;
         if (d.pro_op == PRO_NONE && contiguous) {
-            BulkKernel f = bulk_kernel(d.spec, inv);
+            BulkKernel f = bulk_kernel(d.spec, inv, d.epi_op == EPI_NONE);
             const uint32_t smem = 128 + (d.C * d.R + d.C * d.lane_stride + 1u) * uint32_t(sizeof(vec2_t));
             const int per_sm = f ? prepare((const void*)f, smem) : -1;
             const uint32_t grid = uint32_t(std::max(per_sm, 0)) * uint32_t(sm_count());
-            if (per_sm > 0 && d.tiles >= 2 * grid) {
-                f<<<grid, kPassThreads, smem, st>>>(d, uint32_t(wait_slot()), bulk_wait_polls());
+            uint32_t* fail = wait_flags();
+            if (fail && per_sm > 0 && d.tiles >= 2 * grid) {
+                f<<<grid, kPassThreads, smem, st>>>(d, fail + wait_slot(), bulk_wait_polls());
                 note_cuda_error(cudaGetLastError());
                 note_bulk_launch();
                 count_launch();
@@ -255,7 +288,7 @@ void launch_pass_reg(const PassDesc& d, const PassExtra& x, cudaStream_t st) {
                                        ? d.in_es == 1 && d.lanes_j % 2 == 0 && d.in_bs % 2 == 0
                                        : d.in_bs == 1 && d.in_es % 2 == 0 && d.batch % 2 == 0;
             const bool pairs = rows_even && (reinterpret_cast<uintptr_t>(d.in) & 15u) == 0;
-            AsyncKernel f = async_kernel(d.spec, inv);
+            AsyncKernel f = async_kernel(d.spec, inv, d.epi_op == EPI_NONE);
             const uint32_t smem =
                 (d.C * d.R + d.C * d.lane_stride + 1u) * uint32_t(sizeof(vec2_t));
             const int per_sm = f ? prepare((const void*)f, smem) : -1;
@@ -293,8 +326,10 @@ void launch_pass_reg(const PassDesc& d, const PassExtra& x, cudaStream_t st) {
 }
 #endif
 
+#endif
 }  // namespace kfft
 
+#if KFFT_REG_PART == 0
 extern "C" {
 // Test hook: polls a bulk-copy wait makes before it gives up (0 restores the
 // default of about a second).  Only a test that checks the failure path
@@ -314,3 +349,4 @@ KFFT_API int kfft_gb300_check_waits(void* stream) {
     return kfft::take_wait_failures(static_cast<cudaStream_t>(stream)) ? 1 : 0;
 }
 }  // extern "C"
+#endif
