@@ -378,8 +378,9 @@ inline CopyRange copy_range(size_t b0, size_t b1, size_t total, bool first, bool
 // Shared-memory slots from one lane to the next in a compile-time
 // (power-of-two) tile body of C lanes of R points run by `threads` threads:
 // the padded lane plus the skew with the fewest bank conflicts.
+// With `linear` (the tile's radices) the same for a tile without padding.
 uint32_t spec_lane_stride(uint32_t R, uint32_t C, bool load_lane, bool store_lane,
-                          uint32_t threads);
+                          uint32_t threads, const std::vector<uint8_t>* linear = nullptr);
 // true when every pass of a direct plan run down the columns of a row-major
 // array gets tiles of four columns or more (32-byte row segments)
 bool columns_coalesce(const FftPlan& P);

@@ -243,10 +243,15 @@ struct OddAcc {
                                                vec2_t& b) {
         constexpr real_t cc = real_t(trig_ratio(long(N) * K, P, false));
         constexpr real_t ss = real_t(trig_ratio(long(N) * K, P, true));
+#if defined(KFFT_HALF_SCALAR)
+        a = __ffma2_rn(s[N - 1], make_float2(cc, cc), a);
+        b = __ffma2_rn(d[N - 1], make_float2(ss, ss), b);
+#else
         a.x += s[N - 1].x * cc;
         a.y += s[N - 1].y * cc;
         b.x += d[N - 1].x * ss;
         b.y += d[N - 1].y * ss;
+#endif
         if constexpr (N < H) OddAcc<P, K, N + 1, H>::run(s, d, a, b);
     }
 };
@@ -763,10 +768,10 @@ __device__ __forceinline__ void fused_store(const PassDesc& d, uint32_t bs, uint
     const uint32_t ko = j - blo * d.Ns;
     const uint32_t base = blo * d.Ns * d.R + ko;
     if (STORE == STORE_PLAIN || (STORE == STORE_ANY && d.epi_op == EPI_NONE)) {
-        vec2_t* o = d.out + uint64_t(bs) * d.out_bs;
-        const uint64_t es = d.out_es;
+        vec2_t* o = d.out + uint64_t(bs) * d.out_bs + uint64_t(base + ob * d.Ns) * d.out_es;
+        const uint64_t step = uint64_t(ns * d.Ns) * d.out_es;
 #pragma unroll
-        for (int q = 0; q < P; ++q) o[uint64_t(base + (ob + q * ns) * d.Ns) * es] = cscale(v[q], d.scale);
+        for (int q = 0; q < P; ++q) o[q * step] = cscale(v[q], d.scale);
     } else if (STORE == STORE_PRODUCT && d.epi_op == EPI_RADER_INV) {
         constexpr int G = P < 8 ? P : 8;
         const uint32_t k = base + ob * d.Ns, ks = ns * d.Ns;
@@ -823,11 +828,18 @@ __device__ __forceinline__ void fused_store(const PassDesc& d, uint32_t bs, uint
 // butterfly at a time from `src` (global memory on the first pass, else a
 // shared buffer) and writes it to `dst` (global memory on the last pass, else
 // the other shared buffer).
-template <int P, bool INV>
+// LIN: element i of a lane lies at slot i of its shared-memory lane (run-time
+// FP32 tiles: an address is a base plus q steps), else at pad(i).
+template <bool LIN>
+__device__ __forceinline__ uint32_t slot(uint32_t i) {
+    return LIN ? i : pad(i);
+}
+
+template <int P, bool INV, int STORE, bool LIN>
 __device__ __forceinline__ void fused_pass(const PassDesc& d, const InnerStep& st,
                                            const vec2_t* src, vec2_t* dst, uint32_t lane0,
                                            uint32_t total, int sio, int dio) {
-    const uint32_t m = st.m;
+    const uint32_t m = st.m, ns = st.ns;
     const uint32_t items = d.C * m;
     const bool cfast = (sio == IO_GLOBAL) ? (d.load_mode == MODE_LANE)
                                           : ((dio == IO_GLOBAL) ? (d.store_mode == MODE_LANE) : false);
@@ -873,7 +885,7 @@ __device__ __forceinline__ void fused_pass(const PassDesc& d, const InnerStep& s
             }
         } else {
 #pragma unroll
-            for (int q = 0; q < P; ++q) v[q] = src[c * d.lane_stride + pad(jj + q * m)];
+            for (int q = 0; q < P; ++q) v[q] = src[c * d.lane_stride + slot<LIN>(jj + q * m)];
         }
         const uint32_t blk = fdiv(jj, st.div_ns);
         const uint32_t kk = jj - blk * st.ns;
@@ -886,9 +898,9 @@ __device__ __forceinline__ void fused_pass(const PassDesc& d, const InnerStep& s
 #endif
         if (dio == IO_SMEM) {
 #pragma unroll
-            for (int q = 0; q < P; ++q) dst[c * d.lane_stride + pad(ob + q * st.ns)] = v[q];
+            for (int q = 0; q < P; ++q) dst[c * d.lane_stride + slot<LIN>(ob + q * ns)] = v[q];
         } else if (live) {
-            fused_store<P>(d, bs, j, ob, st.ns, v);
+            fused_store<P, STORE>(d, bs, j, ob, ns, v);
         }
     }
 }
@@ -1571,26 +1583,26 @@ __device__ __forceinline__ void tile_loop_bulk(const PassDesc& d, unsigned char*
 }
 #endif
 
-template <bool INV>
+template <bool INV, int STORE, bool LIN>
 __device__ __forceinline__ void fused_dispatch(int P, const PassDesc& d, const InnerStep& st,
                                                const vec2_t* src, vec2_t* dst, uint32_t lane0,
                                                uint32_t total, int sio, int dio) {
     switch (P) {
-        case 2: fused_pass<2, INV>(d, st, src, dst, lane0, total, sio, dio); break;
-        case 3: fused_pass<3, INV>(d, st, src, dst, lane0, total, sio, dio); break;
-        case 4: fused_pass<4, INV>(d, st, src, dst, lane0, total, sio, dio); break;
-        case 5: fused_pass<5, INV>(d, st, src, dst, lane0, total, sio, dio); break;
-        case 7: fused_pass<7, INV>(d, st, src, dst, lane0, total, sio, dio); break;
-        case 6: fused_pass<6, INV>(d, st, src, dst, lane0, total, sio, dio); break;
-        case 8: fused_pass<8, INV>(d, st, src, dst, lane0, total, sio, dio); break;
-        case 9: fused_pass<9, INV>(d, st, src, dst, lane0, total, sio, dio); break;
-        case 10: fused_pass<10, INV>(d, st, src, dst, lane0, total, sio, dio); break;
-        case 11: fused_pass<11, INV>(d, st, src, dst, lane0, total, sio, dio); break;
-        case 12: fused_pass<12, INV>(d, st, src, dst, lane0, total, sio, dio); break;
-        case 13: fused_pass<13, INV>(d, st, src, dst, lane0, total, sio, dio); break;
-        case 14: fused_pass<14, INV>(d, st, src, dst, lane0, total, sio, dio); break;
-        case 15: fused_pass<15, INV>(d, st, src, dst, lane0, total, sio, dio); break;
-        case 16: fused_pass<16, INV>(d, st, src, dst, lane0, total, sio, dio); break;
+        case 2: fused_pass<2, INV, STORE, LIN>(d, st, src, dst, lane0, total, sio, dio); break;
+        case 3: fused_pass<3, INV, STORE, LIN>(d, st, src, dst, lane0, total, sio, dio); break;
+        case 4: fused_pass<4, INV, STORE, LIN>(d, st, src, dst, lane0, total, sio, dio); break;
+        case 5: fused_pass<5, INV, STORE, LIN>(d, st, src, dst, lane0, total, sio, dio); break;
+        case 7: fused_pass<7, INV, STORE, LIN>(d, st, src, dst, lane0, total, sio, dio); break;
+        case 6: fused_pass<6, INV, STORE, LIN>(d, st, src, dst, lane0, total, sio, dio); break;
+        case 8: fused_pass<8, INV, STORE, LIN>(d, st, src, dst, lane0, total, sio, dio); break;
+        case 9: fused_pass<9, INV, STORE, LIN>(d, st, src, dst, lane0, total, sio, dio); break;
+        case 10: fused_pass<10, INV, STORE, LIN>(d, st, src, dst, lane0, total, sio, dio); break;
+        case 11: fused_pass<11, INV, STORE, LIN>(d, st, src, dst, lane0, total, sio, dio); break;
+        case 12: fused_pass<12, INV, STORE, LIN>(d, st, src, dst, lane0, total, sio, dio); break;
+        case 13: fused_pass<13, INV, STORE, LIN>(d, st, src, dst, lane0, total, sio, dio); break;
+        case 14: fused_pass<14, INV, STORE, LIN>(d, st, src, dst, lane0, total, sio, dio); break;
+        case 15: fused_pass<15, INV, STORE, LIN>(d, st, src, dst, lane0, total, sio, dio); break;
+        case 16: fused_pass<16, INV, STORE, LIN>(d, st, src, dst, lane0, total, sio, dio); break;
         default: break;
     }
 }
@@ -1603,12 +1615,17 @@ __device__ __forceinline__ void fused_dispatch(int P, const PassDesc& d, const I
 // the pass kernel launches those as kernels of their own and leaves it off.
 // TC: keep the tensor-core radix-16 stage; the queue kernel leaves it off
 // (its planner clears d.tc) to keep its instruction footprint small.
-template <bool INV, bool SPEC = true, bool TC = true>
+template <bool INV, bool SPEC = true, bool TC = true, int STORE = STORE_ANY>
 __device__ __forceinline__ void tile_body_reg(const PassDesc& d, const PassExtra& x, uint32_t tile,
                                               vec2_t* sm) {
     const uint32_t total = d.batch * d.lanes_j;
     const uint32_t lane0 = tile * d.C;
     const int np = d.nrad;
+#if defined(KFFT_HALF_SCALAR)
+    constexpr bool kLin = !TC;  // (the tensor-core stage keeps the padded slots)
+#else
+    constexpr bool kLin = false;
+#endif
     if (np == 0) {  // length-1 sub-FFT: the pass is a scaled copy (with its fused ops)
         for (uint32_t c = threadIdx.x; c < d.C; c += blockDim.x) {
             const uint32_t g = lane0 + c;
@@ -1661,8 +1678,11 @@ __device__ __forceinline__ void tile_body_reg(const PassDesc& d, const PassExtra
             tc_pass16<INV>(d, x.step[p], src, dst, lane0, total, sio, dio, Fr, Fi, Gm);
         else
 #endif
-            fused_dispatch<INV>(d.rad[p], d, x.step[p], src, dst, lane0, total, sio, dio);
-        if (!last) __syncthreads();
+            fused_dispatch<INV, STORE, kLin>(d.rad[p], d, x.step[p], src, dst, lane0, total, sio, dio);
+        // (also after the last stage: a barrier that depends on `last` makes the
+        // compiler spill the values of every radix around it; with the
+        // tensor-core stage it is the other way round)
+        if (!TC || !last) __syncthreads();
         src = dst;
     }
 }

@@ -138,12 +138,20 @@ BulkKernel bulk_kernel(uint32_t spec, bool inv, bool plain) {
 
 #if KFFT_REG_PART == 0
 #if defined(KFFT_HALF_SCALAR)
-template <bool INV>
-__global__ void __launch_bounds__(kPassThreads, KFFT_REG_MINBLOCKS) k_pass_reg(const __grid_constant__ PassDesc d,
+// The run-time tile: bound by instruction issue and latency (108 thread
+// instructions a point for 10 x 10 x 10 before, at two instructions a clock).
+// Apart from the tensor-core stage and the product stores, with the elements
+// of a lane side by side in shared memory (no padding arithmetic), packed
+// odd-radix sums and no spills it fits 64 registers, four CTAs an SM.  2^24
+// points forward, us, before -> three CTAs -> four: length 1000 96 -> 79 -> 79,
+// 1080 117 -> 76 -> 80, 2187 131 -> 114 -> 99, 3003 93 -> 81 -> 73, 59049
+// 221 -> 200 -> 169; a 4160^2 convolution 597 -> 532 -> 478.
+template <bool INV, int STORE, bool TC, int BLOCKS>
+__global__ void __launch_bounds__(kPassThreads, BLOCKS) k_pass_reg(const __grid_constant__ PassDesc d,
                                                               const __grid_constant__ PassExtra x) {
     extern __shared__ __align__(16) unsigned char smem_raw[];
     // power-of-two FP32 passes launch k_pass_spec / k_pass_pipe instead
-    tile_body_reg<INV, false>(d, x, blockIdx.x, reinterpret_cast<vec2_t*>(smem_raw));
+    tile_body_reg<INV, false, TC, STORE>(d, x, blockIdx.x, reinterpret_cast<vec2_t*>(smem_raw));
 }
 
 // Set when a bulk-copy wait of k_pass_bulk ran out (only a failed or very
@@ -246,7 +254,11 @@ void launch_pass_reg(const PassDesc& d, const PassExtra& x, cudaStream_t st) {
     // one-time shared-memory limit of the generic kernels (thread-safe; a
     // failure is reported on every call)
     static const cudaError_t configured = [] {
-        for (const void* f : {(const void*)k_pass_reg<false>, (const void*)k_pass_reg<true>}) {
+        for (const void* f :
+             {(const void*)k_pass_reg<false, STORE_PLAIN, false, 4>, (const void*)k_pass_reg<true, STORE_PLAIN, false, 4>,
+              (const void*)k_pass_reg<false, STORE_PRODUCT, false, 4>,
+              (const void*)k_pass_reg<true, STORE_PRODUCT, false, 4>,
+              (const void*)k_pass_reg<false, STORE_ANY, true, 3>, (const void*)k_pass_reg<true, STORE_ANY, true, 3>}) {
             cudaError_t e = cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                                  227 * 1024);
             if (e != cudaSuccess) {
@@ -319,8 +331,13 @@ void launch_pass_reg(const PassDesc& d, const PassExtra& x, cudaStream_t st) {
             return;
         }
     }
-    if (d.inv) k_pass_reg<true><<<d.tiles, d.threads, d.smem_bytes, st>>>(d, x);
-    else k_pass_reg<false><<<d.tiles, d.threads, d.smem_bytes, st>>>(d, x);
+    // the tensor-core stages, the plain store and the product stores each have
+    // a kernel of their own (smaller, and no registers held for the others)
+    void (*f)(PassDesc, PassExtra);
+    if (d.tc) f = d.inv ? k_pass_reg<true, STORE_ANY, true, 3> : k_pass_reg<false, STORE_ANY, true, 3>;
+    else if (d.epi_op == EPI_NONE) f = d.inv ? k_pass_reg<true, STORE_PLAIN, false, 4> : k_pass_reg<false, STORE_PLAIN, false, 4>;
+    else f = d.inv ? k_pass_reg<true, STORE_PRODUCT, false, 4> : k_pass_reg<false, STORE_PRODUCT, false, 4>;
+    f<<<d.tiles, d.threads, d.smem_bytes, st>>>(d, x);
     note_cuda_error(cudaGetLastError());
     count_launch();
 }

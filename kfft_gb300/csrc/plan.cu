@@ -78,15 +78,17 @@ static uint32_t smem_for(uint32_t elems) {
 // in plan_host.h), cached per (R, C, lane modes, threads)
 // ---------------------------------------------------------------------------
 uint32_t spec_lane_stride(uint32_t R, uint32_t C, bool load_lane, bool store_lane,
-                          uint32_t threads) {
+                          uint32_t threads, const std::vector<uint8_t>* linear) {
     static std::mutex mu;
     static std::map<std::pair<uint64_t, uint32_t>, uint32_t> cache;
     const auto key = std::make_pair((uint64_t(R) << 32) | C,
-                                    uint32_t(load_lane) | (uint32_t(store_lane) << 1) | (threads << 2));
+                                    uint32_t(load_lane) | (uint32_t(store_lane) << 1) |
+                                        (uint32_t(linear != nullptr) << 2) | (threads << 3));
     std::lock_guard<std::mutex> lk(mu);
     auto it = cache.find(key);
     if (it != cache.end()) return it->second;
-    const uint32_t best = lane_stride_search(R, C, load_lane, store_lane, threads);
+    const uint32_t best = linear ? linear_stride_search(*linear, R, C, load_lane, store_lane, threads)
+                                 : lane_stride_search(R, C, load_lane, store_lane, threads);
     cache[key] = best;
     return best;
 }
@@ -231,6 +233,9 @@ static bool build_direct(FftPlan* P, DeviceArena& arena, cudaStream_t st) {
         s.R = R;
         s.Ns = Ns;
         s.radices = inner_radices(R);
+#if defined(KFFT_HALF_SCALAR)
+        if (R & (R - 1)) s.radices = linear_radices(s.radices);
+#endif
         if (s.radices.size() > size_t(kMaxInnerRadices)) return false;
         auto it = inner.find(R);
         if (it == inner.end()) {
@@ -650,8 +655,14 @@ static PassDesc make_desc(const FftPlan& P, size_t pi, const vec2_t* in, const L
         d.fx = d.nrad > 0 ? 1 : 0;
         if (d.spec) d.threads = std::max<uint32_t>(32, (elems / 8 + 31) / 32 * 32);
 #endif
+#if defined(KFFT_HALF_SCALAR)
+        const bool linear = !d.spec && !d.tc;
+#else
+        const bool linear = false;
+#endif
         d.lane_stride = spec_lane_stride(s.R, C, d.load_mode == MODE_LANE,
-                                         d.store_mode == MODE_LANE, kPassThreads);
+                                         d.store_mode == MODE_LANE, kPassThreads,
+                                         linear ? &s.radices : nullptr);
         d.smem_bytes = nbuf * (C * d.lane_stride + 1u) * uint32_t(sizeof(vec2_t));
 #if !defined(KFFT_HALF_SCALAR)
         d.fx_words = d.smem_bytes;

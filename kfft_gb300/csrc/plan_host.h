@@ -250,10 +250,12 @@ inline uint32_t smem_wavefronts(const int64_t* idx) {
 // by `threads` threads).  Stages with a global access in lane mode put
 // consecutive threads on consecutive lanes; the others put them on
 // consecutive butterflies of one lane.
-inline uint64_t tile_smem_cost(uint32_t R, uint32_t C, uint32_t stride, bool load_lane,
-                               bool store_lane, uint32_t threads) {
-    auto padh = [](uint64_t i) { return i + i / kRowElems; };
-    const std::vector<uint8_t> rad = inner_radices(R);
+// `linear`: element i of a lane at slot i (run-time FP32 tiles), without the
+// padding slot per 128 bytes.
+inline uint64_t tile_smem_cost(const std::vector<uint8_t>& rad, uint32_t R, uint32_t C,
+                               uint32_t stride, bool load_lane, bool store_lane, uint32_t threads,
+                               bool linear) {
+    auto padh = [&](uint64_t i) { return linear ? i : i + i / kRowElems; };
     const size_t np = rad.size();
     uint64_t cost = 0;
     uint32_t NS = 1;
@@ -292,6 +294,44 @@ inline uint64_t tile_smem_cost(uint32_t R, uint32_t C, uint32_t stride, bool loa
         NS *= P;
     }
     return cost;
+}
+
+inline uint64_t tile_smem_cost(uint32_t R, uint32_t C, uint32_t stride, bool load_lane,
+                               bool store_lane, uint32_t threads) {
+    return tile_smem_cost(inner_radices(R), R, C, stride, load_lane, store_lane, threads, false);
+}
+
+// Radices of a linear tile: the one whose outputs (the first stage writes P
+// consecutive slots a butterfly) spread over the banks best comes first.
+inline std::vector<uint8_t> linear_radices(std::vector<uint8_t> rad) {
+    auto shared = [](uint32_t p) {  // common power of two with the 16 slots of a row
+        uint32_t g = 1;
+        while (g < 16 && p % (2 * g) == 0) g *= 2;
+        return g;
+    };
+    size_t best = 0;
+    for (size_t i = 1; i < rad.size(); ++i)
+        if (shared(rad[i]) < shared(rad[best])) best = i;
+    if (best) std::rotate(rad.begin(), rad.begin() + best, rad.begin() + best + 1);
+    return rad;
+}
+
+// Lane stride of a linear tile: the lane length plus the skew with the fewest
+// wavefronts.
+inline uint32_t linear_stride_search(const std::vector<uint8_t>& rad, uint32_t R, uint32_t C,
+                                     bool load_lane, bool store_lane, uint32_t threads) {
+    uint32_t best = R;
+    uint64_t best_cost = ~uint64_t(0);
+    if (C > 1 && rad.size() > 1) {
+        for (uint32_t skew = 0; skew < kRowElems; ++skew) {
+            const uint64_t c = tile_smem_cost(rad, R, C, R + skew, load_lane, store_lane, threads, true);
+            if (c < best_cost) {
+                best_cost = c;
+                best = R + skew;
+            }
+        }
+    }
+    return best;
 }
 
 // The padded lane length plus the skew (0 .. kRowElems-1 slots) with the

@@ -63,3 +63,29 @@ def test_contiguous_batches(libf, n):
     ref = np.fft.fft(x[-8:].astype(np.complex128), axis=1)
     assert rel_l2(y[-8:], ref) <= TOL32
     assert rel_l2(y[:8], np.fft.fft(x[:8].astype(np.complex128), axis=1)) <= TOL32
+
+
+# run-time tiles: every radix in the first place and behind others, one, two
+# and more stages, and (through Bluestein and a convolution) the product stores
+@pytest.mark.parametrize("n", [3, 5, 6, 7, 9, 10, 11, 12, 13, 14, 15, 24, 36, 60, 105, 169, 196, 225, 240,
+                               1000, 1080, 1155, 1728, 1920, 2016, 2187, 2197, 2310, 3003, 3375, 4000, 4095,
+                               4160, 59049, 100000, 1009, 4111])
+def test_run_time_tiles(libf, n):
+    batch = max(3, 20000 // n)
+    rng = np.random.default_rng(n)
+    x = (rng.standard_normal((batch, n), np.float32) + 1j * rng.standard_normal((batch, n), np.float32)).astype(np.complex64)
+    y = libf.fft_cpx(x)
+    assert rel_l2(y, np.fft.fft(x.astype(np.complex128), axis=1)) <= TOL32
+    z = libf.fft_cpx(x, K.FLAG_INVERSE)
+    assert rel_l2(z, np.fft.ifft(x.astype(np.complex128), axis=1)) <= TOL32
+
+
+@pytest.mark.parametrize("y,x", [(52, 80), (90, 182), (128, 100), (75, 64)])
+def test_run_time_tiles_convolve(libf, y, x):
+    rng = np.random.default_rng(y * x)
+    a, b = (rng.uniform(0, 1, (y, x)).astype(np.float32) for _ in range(2))
+    ref = np.fft.ifft2(np.fft.fft2(a.astype(float)) * np.fft.fft2(b.astype(float))).real
+    got = libf.conv2_scalar(a, b)
+    assert rel_l2(got, ref * (1 if y % 2 else 2)) <= TOL32
+    c = libf.conv2_cpx(a.astype(np.complex64), b.astype(np.complex64))
+    assert rel_l2(c, ref) <= TOL32
