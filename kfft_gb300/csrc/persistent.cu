@@ -8,12 +8,6 @@
 
 namespace kfft {
 
-// 1: publish a finished item with one release add by thread 0 after the
-// CTA's barrier; 0: every thread fences before the barrier and thread 0 adds
-// (uneven FP32 batch: 9.10 against 9.38 ms; FP64 unchanged)
-#ifndef KFFT_QUEUE_RELEASE_ONE
-#define KFFT_QUEUE_RELEASE_ONE 1
-#endif
 // resident CTAs per SM of the queue kernel (its tiles are capped at 2048
 // points): four for FP32 (64 registers a thread), three for the double build
 // (80 registers; 256 sequences of up to 2^18 points 0.89 ms, two CTAs 0.95,
@@ -25,28 +19,17 @@ namespace kfft {
 #define KFFT_QUEUE_MINBLOCKS 3
 #endif
 #endif
-// 1: each CTA claims its items two ahead and copies the next item's record
-// into shared memory while the current one runs; 0: one claim ahead, the
-// record read when its turn comes (uneven FP32 batch: 8.93 against 9.13 ms;
-// FP64 unchanged)
-#ifndef KFFT_QUEUE_PREFETCH
-#define KFFT_QUEUE_PREFETCH 1
-#endif
 
+// Publishes a finished item: the CTA's stores are ordered before one thread's
+// by the barrier, and that thread publishes them all with one release add at
+// GPU scope (the waiting CTA's acquire load pairs with it).  A thread of the
+// last warp does it, so that thread 0 goes on to the next item's dependency
+// meanwhile (512 sequences FP32 1412 -> 1354 us, 256 in double 852 -> 841).
 __device__ __forceinline__ void publish_done(uint32_t* done) {
-#if KFFT_QUEUE_RELEASE_ONE
-    // the CTA's stores are ordered before thread 0's by the barrier, and
-    // thread 0 publishes them all with one release add at GPU scope (the
-    // waiting CTA's acquire load pairs with it)
     __syncthreads();
-    if (threadIdx.x == 0) {
+    if (threadIdx.x == blockDim.x - 32) {
         asm volatile("red.release.gpu.global.add.u32 [%0], %1;" ::"l"(done), "r"(1u) : "memory");
     }
-#else
-    __threadfence();
-    __syncthreads();
-    if (threadIdx.x == 0) atomicAdd(done, 1u);
-#endif
 }
 
 // Thread 0's dependency wait for item q (a bounded spin that sets the error
@@ -59,14 +42,25 @@ __device__ __forceinline__ void item_wait(const QueueItem& q, const uint32_t* do
     *s_ok = ok ? 1u : 0u;
 }
 
-// stage the descriptor in shared memory: one coalesced copy per item, then
-// broadcast reads (measured 14% faster on the uneven batch than reading every
-// field from global memory through L1)
-__device__ __forceinline__ void stage_desc(const PassDesc* __restrict__ descs, uint32_t desc,
-                                           PassDesc* s_desc) {
-    const uint32_t* src = reinterpret_cast<const uint32_t*>(&descs[desc]);
-    uint32_t* dst = reinterpret_cast<uint32_t*>(s_desc);
-    for (uint32_t i = threadIdx.x; i < sizeof(PassDesc) / 4; i += blockDim.x) dst[i] = src[i];
+// Starts copying the descriptor and the stage table of pass `desc` into shared
+// memory (8 bytes a thread and step).  One item ahead, so neither is waited
+// for: 512 sequences FP32 1486 -> 1412 us against copying the descriptor when
+// the item's turn came and reading the stage table from global memory.
+__device__ __forceinline__ void stage_desc(const PassDesc* __restrict__ descs,
+                                           const PassExtra* __restrict__ extras, uint32_t desc,
+                                           PassDesc* s_desc, PassExtra* s_extra) {
+    static_assert(sizeof(PassDesc) % 8 == 0 && sizeof(PassExtra) % 8 == 0, "copied 8 bytes at a time");
+    constexpr uint32_t n0 = sizeof(PassDesc) / 8, n1 = sizeof(PassExtra) / 8;
+    const char* g0 = reinterpret_cast<const char*>(&descs[desc]);
+    const char* g1 = reinterpret_cast<const char*>(&extras[desc]);
+    const uint32_t a0 = uint32_t(__cvta_generic_to_shared(s_desc));
+    const uint32_t a1 = uint32_t(__cvta_generic_to_shared(s_extra));
+    for (uint32_t i = threadIdx.x; i < n0 + n1; i += blockDim.x) {
+        const bool first = i < n0;
+        const char* g = first ? g0 + 8 * i : g1 + 8 * (i - n0);
+        const uint32_t a = first ? a0 + 8 * i : a1 + 8 * (i - n0);
+        asm volatile("cp.async.ca.shared.global [%0], [%1], 8;" ::"r"(a), "l"(g) : "memory");
+    }
 }
 
 __device__ __forceinline__ void run_item(const PassDesc& d, const PassExtra& x, uint32_t tile,
@@ -100,13 +94,14 @@ __global__ void __launch_bounds__(KFFT_QUEUE_THREADS, KFFT_QUEUE_MINBLOCKS) k_pe
     uint32_t* error, uint32_t max_polls) {
     extern __shared__ __align__(16) unsigned char smem_raw[];
     __shared__ uint32_t s_ok;
-    __shared__ __align__(16) PassDesc s_desc;
+    __shared__ __align__(16) PassDesc s_desc[2];
+    __shared__ __align__(16) PassExtra s_extra[2];
     vec2_t* buf = reinterpret_cast<vec2_t*>(smem_raw);
-#if KFFT_QUEUE_PREFETCH
     // Items claimed two ahead, their records in a ring of three shared slots:
     // the current item, the next one (copied in during the previous item)
-    // and the one after it (copied in during this item).  A CTA's claims
-    // increase, so its current item is the earliest of its claims; the
+    // and the one after it (copied in during this item); the next item's
+    // descriptor and stage table are copied in during this one too.  A CTA's
+    // claims increase, so its current item is the earliest of its claims; the
     // earliest claimed and unfinished item of all then is some CTA's current
     // item, whose dependencies (earlier queue positions, all claimed) are
     // done: the queue cannot deadlock.
@@ -123,12 +118,15 @@ __global__ void __launch_bounds__(KFFT_QUEUE_THREADS, KFFT_QUEUE_MINBLOCKS) k_pe
         claim = atomicAdd(head, 1u);
     }
     __syncthreads();
-    uint32_t slot = 0;
+    uint32_t slot = 0, cur = 0;
+    if (s_item[0].desc != kEnd) stage_desc(descs, extras, s_item[0].desc, &s_desc[0], &s_extra[0]);
+    asm volatile("cp.async.wait_all;" ::: "memory");
     while (true) {
         const QueueItem q = s_item[slot];
         if (q.desc == kEnd) break;
+        const uint32_t next = s_item[slot == 2 ? 0u : slot + 1u].desc;
+        if (next != kEnd) stage_desc(descs, extras, next, &s_desc[cur ^ 1], &s_extra[cur ^ 1]);
         if (threadIdx.x == 0) {
-            item_wait(q, done, error, max_polls, &s_ok);
             // the slot the previous item used (every thread read it before
             // the previous item's barriers) takes the record at `claim`
             const uint32_t s2 = slot == 0 ? 2u : slot - 1u;
@@ -139,41 +137,18 @@ __global__ void __launch_bounds__(KFFT_QUEUE_THREADS, KFFT_QUEUE_MINBLOCKS) k_pe
             } else {
                 s_item[s2].desc = kEnd;
             }
-            asm volatile("cp.async.commit_group;" ::: "memory");
+            item_wait(q, done, error, max_polls, &s_ok);
             claim = atomicAdd(head, 1u);
         }
-        stage_desc(descs, q.desc, &s_desc);
         __syncthreads();
-        if (s_ok) run_item(s_desc, extras[q.desc], q.tile, buf);
-        // the next item's record (the group before this item's) has landed
-        if (threadIdx.x == 0) asm volatile("cp.async.wait_group 1;" ::: "memory");
+        if (s_ok) run_item(s_desc[cur], s_extra[cur], q.tile, buf);
+        // the next item's record, descriptor and stage table have landed
+        asm volatile("cp.async.wait_all;" ::: "memory");
         publish_done(&done[q.desc]);
         slot = slot == 2 ? 0u : slot + 1u;
+        cur ^= 1u;
     }
-    if (threadIdx.x == 0) asm volatile("cp.async.wait_all;" ::: "memory");
-#else
-    __shared__ uint32_t s_next;
-    // Each CTA claims its next item while the current one runs, so the
-    // claim's round trip to L2 overlaps work.  This cannot deadlock: the item
-    // of least queue position among those claimed and not finished has every
-    // dependency (an earlier position) done or in a run of its own.
-    if (threadIdx.x == 0) s_next = atomicAdd(head, 1u);
-    __syncthreads();
-    while (true) {
-        const uint32_t it = s_next;
-        __syncthreads();  // every thread has read s_next before it changes
-        if (it >= nitems) return;
-        const QueueItem q = items[it];
-        if (threadIdx.x == 0) {
-            s_next = atomicAdd(head, 1u);
-            item_wait(q, done, error, max_polls, &s_ok);
-        }
-        stage_desc(descs, q.desc, &s_desc);
-        __syncthreads();
-        if (s_ok) run_item(s_desc, extras[q.desc], q.tile, buf);
-        publish_done(&done[q.desc]);
-    }
-#endif
+    asm volatile("cp.async.wait_all;" ::: "memory");
 }
 
 bool launch_persistent(const PassDesc* descs, const void* extras,

@@ -100,7 +100,7 @@ def test_queue_tiles(lib):
     """The queue kernel's tiles: every power of two it runs in one tile, and
     lengths whose stages take one round of its threads or more."""
     lengths = np.array([16, 32, 64, 128, 256, 512, 1024, 2048, 4096, 1 << 17, 11, 1792, 1820, 1848,
-                        1960, 2016, 2028, 2047, 1890, 1331, 2197, 30030, 4099, 65537, 9973], np.uint32)
+                        1960, 2016, 2028, 2047, 1890, 1331, 2197, 30030, 4099, 65537, 9973, 504 * 488, 2016 * 45], np.uint32)
     rng = np.random.default_rng(3)
     x = rng.standard_normal(int(lengths.sum())) + 1j * rng.standard_normal(int(lengths.sum()))
     for flags, f in ((0, np.fft.fft), (K.FLAG_INVERSE, np.fft.ifft)):
