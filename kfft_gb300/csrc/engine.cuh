@@ -149,20 +149,19 @@ struct PassDesc {
 
 // ---- device tables -----------------------------------------------------
 #if !defined(KFFT_HALF_SCALAR)
-// Two-limb tables of the fixed-point tiles, exact to a few 2^-62: forward
-// twiddles exp(-2 pi i (i * mult mod n) / n), the chirp of gen_chirp, and a
-// spectrum divided by the power of two *exp (written on the device; its
-// largest part then lies in [1/4, 1/2)).
-void gen_fx_twiddles(FxTw* t, uint32_t count, uint64_t mult, uint32_t n, cudaStream_t st);
-void gen_fx_chirp(FxTw* c, uint32_t count, uint32_t n, int sign, cudaStream_t st);
+// A spectrum in two-limb form, divided by the power of two exp[1] (written on
+// the device; its largest part then lies in [1/4, 1/2)).
 void gen_fx_spectrum(FxTw* t, const vec2_t* spectrum, uint32_t count, int32_t* exp,
                      cudaStream_t st);
 #endif
 // Fills t[i] = exp(sign * 2 pi i * (i * mult mod n) / n) in FP64 for i < count.
+// With `fx` also the forward ones, exp(-2 pi i (i * mult mod n) / n), in two limbs,
+// exact to a few 2^-62 (fixed-point tiles).
 void gen_twiddles(vec2_t* t, uint32_t count, uint64_t mult, uint32_t n, int sign,
-                  cudaStream_t st);
+                  cudaStream_t st, FxTw* fx = nullptr);
 // Bluestein chirp c[k] = exp(sign * i pi (k^2 mod 2n) / n), k < count.
-void gen_chirp(vec2_t* c, uint32_t count, uint32_t n, int sign, cudaStream_t st);
+// With `fx` also in two limbs.
+void gen_chirp(vec2_t* c, uint32_t count, uint32_t n, int sign, cudaStream_t st, FxTw* fx = nullptr);
 // Bluestein filter b[m] = conj(c[|m|]) on the circle of m_len points (zero elsewhere).
 void gen_bluestein_filter(vec2_t* b, const vec2_t* chirp, uint32_t n, uint32_t m_len,
                           cudaStream_t st);
@@ -319,6 +318,9 @@ struct Workspace {
 struct DeviceArena {
     std::vector<void*> blocks;
     size_t bytes = 0;
+    char* cur = nullptr;  // rest of the newest block
+    size_t left = 0;
+    size_t last = 0;      // size step of the newest block
     void* alloc(size_t bytes);
     ~DeviceArena();
 };

@@ -165,16 +165,33 @@ static bool reg_tile_fits(uint32_t R, uint32_t C, uint32_t cap = kRegTile,
 // ---------------------------------------------------------------------------
 // device arena
 // ---------------------------------------------------------------------------
+// Tables are carved out of blocks that double from 16 KB to 4 MB (a plan of many
+// lengths has thousands of tables, and planning a batch of 256 lengths spent
+// most of its time in cudaMalloc); a large table has a block of its own.
 void* DeviceArena::alloc(size_t n) {
+    n = (std::max<size_t>(n, 16) + 255) & ~size_t(255);
+    if (n <= left) {
+        void* p = cur;
+        cur += n;
+        left -= n;
+        return p;
+    }
+    const size_t next = std::min<size_t>(std::max<size_t>(2 * last, size_t(16) << 10), size_t(4) << 20);
+    const size_t size = std::max(n, next);
     void* p = nullptr;
-    cudaError_t e = cudaMalloc(&p, n ? n : 16);
+    cudaError_t e = cudaMalloc(&p, size);
     if (e != cudaSuccess) {
         note_cuda_error(e);
         return nullptr;
     }
     blocks.push_back(p);
-    bytes += n;
-    account_device_bytes(int64_t(n));
+    bytes += size;
+    account_device_bytes(int64_t(size));
+    if (size - n > left) {  // the rest of this block serves the next tables
+        cur = static_cast<char*>(p) + n;
+        left = size - n;
+    }
+    last = next;
     return p;
 }
 
@@ -251,14 +268,14 @@ static bool build_direct(FftPlan* P, DeviceArena& arena, cudaStream_t st) {
         if (it == inner.end()) {
             vec2_t* t = static_cast<vec2_t*>(arena.alloc(sizeof(vec2_t) * R));
             if (!t) return false;
-            gen_twiddles(t, R, 1, R, P->sign, st);
-            it = inner.emplace(R, t).first;
+            FxTw* f = nullptr;
 #if !defined(KFFT_HALF_SCALAR)
-            FxTw* f = static_cast<FxTw*>(arena.alloc(sizeof(FxTw) * R));
+            f = static_cast<FxTw*>(arena.alloc(sizeof(FxTw) * R));
             if (!f) return false;
-            gen_fx_twiddles(f, R, 1, R, st);
             fx_inner[R] = f;
 #endif
+            gen_twiddles(t, R, 1, R, P->sign, st, f);
+            it = inner.emplace(R, t).first;
         }
         s.tw_inner = it->second;
 #if !defined(KFFT_HALF_SCALAR)
@@ -276,17 +293,16 @@ static bool build_direct(FftPlan* P, DeviceArena& arena, cudaStream_t st) {
         vec2_t* lo = static_cast<vec2_t*>(arena.alloc(sizeof(vec2_t) * nlo));
         vec2_t* hi = static_cast<vec2_t*>(arena.alloc(sizeof(vec2_t) * nhi));
         if (!lo || !hi) return false;
-        gen_twiddles(lo, nlo, 1, N, P->sign, st);
-        gen_twiddles(hi, nhi, uint64_t(nlo), N, P->sign, st);
+        FxTw *flo = nullptr, *fhi = nullptr;
 #if !defined(KFFT_HALF_SCALAR)
-        FxTw* flo = static_cast<FxTw*>(arena.alloc(sizeof(FxTw) * nlo));
-        FxTw* fhi = static_cast<FxTw*>(arena.alloc(sizeof(FxTw) * nhi));
+        flo = static_cast<FxTw*>(arena.alloc(sizeof(FxTw) * nlo));
+        fhi = static_cast<FxTw*>(arena.alloc(sizeof(FxTw) * nhi));
         if (!flo || !fhi) return false;
-        gen_fx_twiddles(flo, nlo, 1, N, st);
-        gen_fx_twiddles(fhi, nhi, uint64_t(nlo), N, st);
         P->fx_lo = flo;
         P->fx_hi = fhi;
 #endif
+        gen_twiddles(lo, nlo, 1, N, P->sign, st, flo);
+        gen_twiddles(hi, nhi, uint64_t(nlo), N, P->sign, st, fhi);
         P->tw_lo = lo;
         P->tw_hi = hi;
         P->tw_shift = shift;
@@ -342,24 +358,18 @@ PlanVariant plan_variant(uint32_t index) {
     return v;
 }
 
-// The two-limb forms of a Rader or Bluestein plan's tables (double build).
-static bool fx_tables(FftPlan* P, DeviceArena& arena, int sign, cudaStream_t st) {
+// The two-limb form of a Rader or Bluestein plan's spectrum (double build).
+static bool fx_spectrum(FftPlan* P, DeviceArena& arena, cudaStream_t st) {
 #if defined(KFFT_HALF_SCALAR)
-    (void)P, (void)arena, (void)sign, (void)st;
+    (void)P, (void)arena, (void)st;
     return true;
 #else
     FxTw* f = static_cast<FxTw*>(arena.alloc(sizeof(FxTw) * P->L));
-    int32_t* e = static_cast<int32_t*>(arena.alloc(sizeof(int32_t)));
+    int32_t* e = static_cast<int32_t*>(arena.alloc(2 * sizeof(int32_t)));
     if (!f || !e) return false;
     gen_fx_spectrum(f, P->spectrum, P->L, e, st);
     P->fx_spectrum = f;
-    if (P->chirp) {
-        FxTw* c = static_cast<FxTw*>(arena.alloc(sizeof(FxTw) * P->N));
-        if (!c) return false;
-        gen_fx_chirp(c, P->N, P->N, sign, st);
-        P->fx_chirp = c;
-    }
-    cudaMemcpyAsync(&P->fx_spectrum_e, e, sizeof(int32_t), cudaMemcpyDeviceToHost, st);
+    cudaMemcpyAsync(&P->fx_spectrum_e, e + 1, sizeof(int32_t), cudaMemcpyDeviceToHost, st);
     const cudaError_t r = cudaStreamSynchronize(st);
     if (r != cudaSuccess) note_cuda_error(r);
     return r == cudaSuccess;
@@ -432,7 +442,7 @@ FftPlan* make_plan(uint32_t N, int sign, DeviceArena& arena, cudaStream_t st,
         }
         scale_table(spec, L, 1.0 / double(L), st);
         P->spectrum = spec;
-        if (!fx_tables(P, arena, sign, st)) {
+        if (!fx_spectrum(P, arena, st)) {
             delete P;
             return nullptr;
         }
@@ -459,7 +469,16 @@ FftPlan* make_plan(uint32_t N, int sign, DeviceArena& arena, cudaStream_t st,
         delete P;
         return nullptr;
     }
-    gen_chirp(chirp, N, N, sign, st);
+    FxTw* fx_chirp = nullptr;
+#if !defined(KFFT_HALF_SCALAR)
+    fx_chirp = static_cast<FxTw*>(arena.alloc(sizeof(FxTw) * N));
+    if (!fx_chirp) {
+        delete P;
+        return nullptr;
+    }
+    P->fx_chirp = fx_chirp;
+#endif
+    gen_chirp(chirp, N, N, sign, st, fx_chirp);
     gen_bluestein_filter(filt, chirp, N, uint32_t(M), st);
     P->sub_fwd = make_plan(uint32_t(M), -1, arena, st, max_prime, var);
     P->sub_inv = make_plan(uint32_t(M), +1, arena, st, max_prime, var);
@@ -474,7 +493,7 @@ FftPlan* make_plan(uint32_t N, int sign, DeviceArena& arena, cudaStream_t st,
     scale_table(spec, uint32_t(M), 1.0 / double(M), st);
     P->chirp = chirp;
     P->spectrum = spec;
-    if (!fx_tables(P, arena, sign, st)) {
+    if (!fx_spectrum(P, arena, st)) {
         delete P;
         return nullptr;
     }

@@ -26,7 +26,14 @@ void FastDiv::init(uint32_t div) {
 // ---------------------------------------------------------------------------
 // FP64 table generation
 // ---------------------------------------------------------------------------
-__global__ void k_gen_twiddles(vec2_t* t, uint32_t count, uint64_t mult, uint32_t n, int sign) {
+// two limbs of each part
+__device__ __forceinline__ FxTw fx_tw_of(fx_t re, fx_t im) {
+    return {fx_hi(re), fx_lo(re), fx_hi(im), fx_lo(im)};
+}
+
+// With `fx` (double build) the two-limb forward twiddles of a fixed-point tile
+// are written beside the table.
+__global__ void k_gen_twiddles(vec2_t* t, FxTw* fx, uint32_t count, uint64_t mult, uint32_t n, int sign) {
     for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < count;
          i += gridDim.x * blockDim.x) {
         uint64_t e = (uint64_t(i) * mult) % n;
@@ -34,20 +41,25 @@ __global__ void k_gen_twiddles(vec2_t* t, uint32_t count, uint64_t mult, uint32_
         double s, c;
         sincospi(2.0 * double(es) / double(n), &s, &c);
         t[i] = {real_t(c), real_t(sign * s)};
+        if (fx) {
+            const FxCosSin v = fx_cossin(e, n);
+            fx[i] = fx_tw_of(v.c, -v.s);
+        }
     }
 }
 
 void gen_twiddles(vec2_t* t, uint32_t count, uint64_t mult, uint32_t n, int sign,
-                  cudaStream_t st) {
+                  cudaStream_t st, FxTw* fx) {
     if (!count) return;
     uint32_t blocks = (count + 255) / 256;
     if (blocks > 4096) blocks = 4096;
-    k_gen_twiddles<<<blocks, 256, 0, st>>>(t, count, mult, n, sign);
+    k_gen_twiddles<<<blocks, 256, 0, st>>>(t, fx, count, mult, n, sign);
     note_cuda_error(cudaGetLastError());
     count_launch();
 }
 
-__global__ void k_gen_chirp(vec2_t* c, uint32_t count, uint32_t n, int sign) {
+// With `fx` the chirp in two-limb form beside it.
+__global__ void k_gen_chirp(vec2_t* c, FxTw* fx, uint32_t count, uint32_t n, int sign) {
     for (uint32_t k = blockIdx.x * blockDim.x + threadIdx.x; k < count;
          k += gridDim.x * blockDim.x) {
         const uint64_t two_n = 2 * uint64_t(n);
@@ -57,13 +69,17 @@ __global__ void k_gen_chirp(vec2_t* c, uint32_t count, uint32_t n, int sign) {
         double s, co;
         sincospi(double(es) / double(n), &s, &co);
         c[k] = {real_t(co), real_t(sign * s)};
+        if (fx) {
+            const FxCosSin v = fx_cossin(e, two_n);
+            fx[k] = fx_tw_of(v.c, sign < 0 ? -v.s : v.s);
+        }
     }
 }
 
-void gen_chirp(vec2_t* c, uint32_t count, uint32_t n, int sign, cudaStream_t st) {
+void gen_chirp(vec2_t* c, uint32_t count, uint32_t n, int sign, cudaStream_t st, FxTw* fx) {
     uint32_t blocks = (count + 255) / 256;
     if (blocks > 4096) blocks = 4096;
-    k_gen_chirp<<<blocks, 256, 0, st>>>(c, count, n, sign);
+    k_gen_chirp<<<blocks, 256, 0, st>>>(c, fx, count, n, sign);
     note_cuda_error(cudaGetLastError());
     count_launch();
 }
@@ -144,44 +160,6 @@ void scale_table(vec2_t* t, uint32_t count, double s, cudaStream_t st) {
 // ---------------------------------------------------------------------------
 // two-limb tables of the fixed-point tiles
 // ---------------------------------------------------------------------------
-__device__ __forceinline__ FxTw fx_tw_of(fx_t re, fx_t im) {
-    return {fx_hi(re), fx_lo(re), fx_hi(im), fx_lo(im)};
-}
-
-__global__ void k_gen_fx_twiddles(FxTw* t, uint32_t count, uint64_t mult, uint32_t n) {
-    for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < count;
-         i += gridDim.x * blockDim.x) {
-        const FxCosSin v = fx_cossin((uint64_t(i) * mult) % n, n);
-        t[i] = fx_tw_of(v.c, -v.s);
-    }
-}
-
-void gen_fx_twiddles(FxTw* t, uint32_t count, uint64_t mult, uint32_t n, cudaStream_t st) {
-    if (!count) return;
-    const uint32_t blocks = std::min<uint32_t>((count + 255) / 256, 4096);
-    k_gen_fx_twiddles<<<blocks, 256, 0, st>>>(t, count, mult, n);
-    note_cuda_error(cudaGetLastError());
-    count_launch();
-}
-
-__global__ void k_gen_fx_chirp(FxTw* c, uint32_t count, uint32_t n, int sign) {
-    for (uint32_t k = blockIdx.x * blockDim.x + threadIdx.x; k < count;
-         k += gridDim.x * blockDim.x) {
-        const uint64_t two_n = 2 * uint64_t(n);
-        const uint64_t kk = k % two_n;
-        const FxCosSin v = fx_cossin((kk * kk) % two_n, two_n);
-        c[k] = fx_tw_of(v.c, sign < 0 ? -v.s : v.s);
-    }
-}
-
-void gen_fx_chirp(FxTw* c, uint32_t count, uint32_t n, int sign, cudaStream_t st) {
-    if (!count) return;
-    const uint32_t blocks = std::min<uint32_t>((count + 255) / 256, 4096);
-    k_gen_fx_chirp<<<blocks, 256, 0, st>>>(c, count, n, sign);
-    note_cuda_error(cudaGetLastError());
-    count_launch();
-}
-
 // the largest exponent field of a table's parts
 __global__ void k_fx_table_max(const vec2_t* t, uint32_t count, int32_t* field) {
     int m = 0;
@@ -191,25 +169,24 @@ __global__ void k_fx_table_max(const vec2_t* t, uint32_t count, int32_t* field) 
     m = __reduce_max_sync(0xffffffffu, m);
     if ((threadIdx.x & 31) == 0) atomicMax(field, m);
 }
-__global__ void k_fx_table(FxTw* f, const vec2_t* t, uint32_t count, const int32_t* field) {
+// ... and the table against it: a leading bit at 60 stands for 2^(field - 1023),
+// so the exponent of the table's unit is field - 1021
+__global__ void k_fx_table(FxTw* f, const vec2_t* t, uint32_t count, const int32_t* field, int32_t* exp) {
     const int e = *field ? *field : 4096;
+    if (blockIdx.x == 0 && threadIdx.x == 0) *exp = *field ? *field - 1021 : 0;
     for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < count;
          i += gridDim.x * blockDim.x)
         f[i] = fx_tw_of(fx_from_double(t[i].x, e, 60), fx_from_double(t[i].y, e, 60));
 }
-// from an exponent field to the exponent of the table's unit: a leading bit
-// at 60 stands for 2^(field - 1023)
-__global__ void k_fx_table_exp(int32_t* field) { *field = *field ? *field - 1021 : 0; }
 
 void gen_fx_spectrum(FxTw* t, const vec2_t* spectrum, uint32_t count, int32_t* exp,
                      cudaStream_t st) {
     const uint32_t blocks = std::min<uint32_t>((count + 255) / 256, 1024);
     cudaMemsetAsync(exp, 0, sizeof(int32_t), st);
     k_fx_table_max<<<blocks, 256, 0, st>>>(spectrum, count, exp);
-    k_fx_table<<<blocks, 256, 0, st>>>(t, spectrum, count, exp);
-    k_fx_table_exp<<<1, 1, 0, st>>>(exp);
+    k_fx_table<<<blocks, 256, 0, st>>>(t, spectrum, count, exp, exp + 1);
     note_cuda_error(cudaGetLastError());
-    count_launch(3);
+    count_launch(2);
 }
 #endif
 
