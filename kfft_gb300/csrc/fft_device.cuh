@@ -835,6 +835,38 @@ __device__ __forceinline__ uint32_t slot(uint32_t i) {
     return LIN ? i : pad(i);
 }
 
+#if !defined(KFFT_HALF_SCALAR)
+// A middle stage in one buffer (PassDesc::inplace): at most fx_group(P)
+// butterflies a thread, all read before any is written.  Threads past the
+// last butterfly repeat it without storing.
+template <int P, bool INV>
+__device__ __forceinline__ void exchange_pass(const PassDesc& d, const InnerStep& st, vec2_t* buf) {
+    constexpr int G = int(fx_group(P));
+    const uint32_t m = st.m, items = d.C * m;
+    vec2_t v[G][P];
+    uint32_t lane[G], ob[G];
+#pragma unroll
+    for (int g = 0; g < G; ++g) {
+        const uint32_t it = min(threadIdx.x + g * blockDim.x, items - 1);
+        const uint32_t c = fdiv(it, st.div_m), jj = it - c * m;
+        const uint32_t blk = fdiv(jj, st.div_ns), kk = jj - blk * st.ns;
+        lane[g] = c * d.lane_stride;
+        ob[g] = blk * st.ns * P + kk;
+#pragma unroll
+        for (int q = 0; q < P; ++q) v[g][q] = buf[lane[g] + pad(jj + q * m)];
+        if (st.ns > 1) apply_inner_twiddles<P>(v[g], d.tw_inner, kk * st.twstride);
+        dft<P, INV>(v[g]);
+    }
+    __syncthreads();
+#pragma unroll
+    for (int g = 0; g < G; ++g)
+        if (threadIdx.x + g * blockDim.x < items) {
+#pragma unroll
+            for (int q = 0; q < P; ++q) buf[lane[g] + pad(ob[g] + q * st.ns)] = v[g][q];
+        }
+}
+#endif
+
 template <int P, bool INV, int STORE, bool LIN>
 __device__ __forceinline__ void fused_pass(const PassDesc& d, const InnerStep& st,
                                            const vec2_t* src, vec2_t* dst, uint32_t lane0,
@@ -843,18 +875,13 @@ __device__ __forceinline__ void fused_pass(const PassDesc& d, const InnerStep& s
     const uint32_t items = d.C * m;
     const bool cfast = (sio == IO_GLOBAL) ? (d.load_mode == MODE_LANE)
                                           : ((dio == IO_GLOBAL) ? (d.store_mode == MODE_LANE) : false);
-#if defined(KFFT_HALF_SCALAR)
-    for (uint32_t it = threadIdx.x; it < items; it += blockDim.x) {
-#else
-    // d.inplace (one butterfly a thread, `src` and `dst` one buffer): every
-    // thread meets the barrier between the reads and the writes, those
-    // without a butterfly on a copy of the last one that they do not store
-    const bool exchange = d.inplace && sio == IO_SMEM && dio == IO_SMEM;
-    for (uint32_t i0 = 0; i0 < items; i0 += blockDim.x) {
-        const bool act = i0 + threadIdx.x < items;
-        if (!act && !exchange) break;
-        const uint32_t it = act ? i0 + threadIdx.x : items - 1;
+#if !defined(KFFT_HALF_SCALAR)
+    if (d.inplace && sio == IO_SMEM && dio == IO_SMEM) {
+        exchange_pass<P, INV>(d, st, dst);
+        return;
+    }
 #endif
+    for (uint32_t it = threadIdx.x; it < items; it += blockDim.x) {
         uint32_t c, jj;
         if (cfast) {
             jj = fdiv(it, d.div_C);
@@ -892,10 +919,6 @@ __device__ __forceinline__ void fused_pass(const PassDesc& d, const InnerStep& s
         if (st.ns > 1) apply_inner_twiddles<P>(v, d.tw_inner, kk * st.twstride);
         dft<P, INV>(v);
         const uint32_t ob = blk * st.ns * P + kk;
-#if !defined(KFFT_HALF_SCALAR)
-        if (exchange) __syncthreads();
-        if (!act) break;
-#endif
         if (dio == IO_SMEM) {
 #pragma unroll
             for (int q = 0; q < P; ++q) dst[c * d.lane_stride + slot<LIN>(ob + q * ns)] = v[q];

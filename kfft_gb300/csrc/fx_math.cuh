@@ -45,18 +45,19 @@ struct FxCosSin {
     fx_t c, s;
 };
 
-// angle u * pi/4, u in [0, 1] scaled by 2^62
+// angle u * pi/4, u in [0, 1] scaled by 2^62 (the first terms left out, x^21 / 21!
+// and x^20 / 20!, are below 2^-68)
 __host__ __device__ constexpr FxCosSin fx_taylor(fx_t u) {
     const fx_t x = fx_mul62(u, kFxQuarterPi);
     const fx_t x2 = fx_mul62(x, x);
     fx_t term = x, s = x;
-    for (int k = 1; k < 12; ++k) {
+    for (int k = 1; k < 10; ++k) {
         term = -(fx_mul62(term, x2) / fx_t((2 * k) * (2 * k + 1)));
         s += term;
     }
     term = kFxOne;
     fx_t c = kFxOne;
-    for (int k = 1; k < 12; ++k) {
+    for (int k = 1; k < 10; ++k) {
         term = -(fx_mul62(term, x2) / fx_t((2 * k - 1) * (2 * k)));
         c += term;
     }

@@ -18,6 +18,8 @@ constexpr int fx_spec_radix(uint32_t R, uint32_t NS) {
     return rest == 16 || rest == 4 ? 4 : (rest % 8 == 0 ? 8 : int(rest));
 }
 
+constexpr uint32_t kFxPad = 1u << kPadShift;  // slots between padding slots
+
 // Sum of (2 - shift) over the stages from NS on: the change of a lane's
 // exponent from the first stage's values to the last one's.
 template <uint32_t R, uint32_t NS, int IDX>
@@ -93,10 +95,14 @@ __device__ __forceinline__ void fx_spec_exchange(const PassDesc& d, cfx_t* buf, 
         const uint32_t it = threadIdx.x + g * blockDim.x;
         uint32_t b = it < items ? fx_bits<P>(v[g]) : 0u;
         if (it < items) {
-            cfx_t* o = buf + c[g] * d.lane_stride;
+            // padding keeps the P slots equally far apart where the distance is
+            // whole pad periods, or all of them lie in one
+            constexpr bool kLin = NS % kFxPad == 0 || (NS == 1 && kFxPad % P == 0);
+            constexpr uint32_t kStep = NS + (NS >> kPadShift);
             const uint32_t ob = jj[g] % NS + (jj[g] / NS) * (NS * P);
+            cfx_t* o = buf + c[g] * d.lane_stride + (kLin ? pad(ob) : 0u);
 #pragma unroll
-            for (int q = 0; q < P; ++q) o[pad(ob + q * NS)] = v[g][q];
+            for (int q = 0; q < P; ++q) o[kLin ? q * kStep : pad(ob + q * NS)] = v[g][q];
         }
         if (M % 32 == 0 && !lane_mode) {  // the warp's butterflies are all of one lane
             b = __reduce_or_sync(0xffffffffu, b);
@@ -132,9 +138,11 @@ __device__ __forceinline__ void fx_spec_later(const PassDesc& d, cfx_t* buf, uin
             jj[g] = it % M;
         }
         {
-            const cfx_t* s = buf + c[g] * d.lane_stride;
+            constexpr bool kLin = M % kFxPad == 0;
+            constexpr uint32_t kStep = M + (M >> kPadShift);
+            const cfx_t* s = buf + c[g] * d.lane_stride + (kLin ? pad(jj[g]) : 0u);
 #pragma unroll
-            for (int q = 0; q < P; ++q) v[g][q] = s[pad(jj[g] + q * M)];
+            for (int q = 0; q < P; ++q) v[g][q] = s[kLin ? q * kStep : pad(jj[g] + q * M)];
             const int sh = fx_norm(words[IDX * d.C + c[g]], P);
             if (sh >= 0) {
 #pragma unroll
@@ -204,11 +212,18 @@ __device__ __forceinline__ bool fx_spec_tile(const PassDesc& d, uint32_t tile, u
             uint32_t b, j;
             fx_lane(d, lane0 + c[g], b, j);
             const double2* p = d.in + uint64_t(b) * d.in_bs;
+            const uint32_t n0 = j + jj[g] * d.lanes_j;
+            if (d.pro_op == PRO_GATHER) {
 #pragma unroll
-            for (int q = 0; q < P; ++q) {
-                const uint32_t n = j + (jj[g] + q * M) * d.lanes_j;
-                if (d.pro_op == PRO_GATHER) raw[g][q] = __ldcg(&p[uint64_t(__ldg(&d.pro_perm[n])) * d.in_es]);
-                else if (d.pro_op != PRO_CHIRP || n < d.pro_bound) raw[g][q] = __ldcg(&p[uint64_t(n) * d.in_es]);
+                for (int q = 0; q < P; ++q)
+                    raw[g][q] = __ldcg(&p[uint64_t(__ldg(&d.pro_perm[n0 + q * M * d.lanes_j])) * d.in_es]);
+            } else {
+                const uint32_t bound = d.pro_op == PRO_CHIRP ? d.pro_bound : 0xffffffffu;
+                const uint64_t step = uint64_t(M) * d.lanes_j * d.in_es;
+                p += uint64_t(n0) * d.in_es;
+#pragma unroll
+                for (int q = 0; q < P; ++q)
+                    if (n0 + q * M * d.lanes_j < bound) raw[g][q] = __ldcg(&p[q * step]);
             }
         }
     }

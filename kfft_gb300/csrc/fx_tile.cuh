@@ -283,7 +283,7 @@ __device__ __forceinline__ void fx_stage(const PassDesc& d, const InnerStep& st,
             }
             fx_dft<P>(v[g], d.fx_one);
         }
-        if (d.inplace) __syncthreads();
+        __syncthreads();
 #pragma unroll
         for (int g = 0; g < G; ++g) {
             const bool act = base + g * blockDim.x + threadIdx.x < items;

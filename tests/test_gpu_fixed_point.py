@@ -83,12 +83,13 @@ def test_non_finite_values_stay_in_their_sequence(lib, n, what):
     assert not np.any(np.isfinite(y[1]))
 
 
-@pytest.mark.parametrize("n", [9, 64, 1000, 4096, 32768])
+# (216 .. 720: middle stages of several small butterflies a thread)
+@pytest.mark.parametrize("n", [9, 64, 216, 250, 343, 360, 720, 1000, 4096, 32768])
 @pytest.mark.parametrize("e", [-1040, -900, -765, 765, 900])
 def test_ends_of_the_exponent_range(lib, n, e):
     """Scaled by a power of two the transform is the same one, scaled."""
     rng = np.random.default_rng(n)
-    x = rng.standard_normal(n) + 1j * rng.standard_normal(n)
+    x = rng.standard_normal((23, n)) + 1j * rng.standard_normal((23, n))
     got = lib.fft_cpx(x * 2.0 ** (e // 2) * 2.0 ** (e - e // 2))
     ref = lib.fft_cpx(x)
     # below 2^-1022 the inputs themselves lose bits
