@@ -929,10 +929,12 @@ def aggregate_over_ranks(ms_total, flops_per_step, steps, world, dist=None, devi
 # pass launches).  The uneven batch is too large for a full-set capture:
 # every 8th sequence was captured (37.47 M points, 2.708 GB) and scaled by
 # points, which the same length mix allows.
+# (The double queue's figure is of its FP64 tiles; its fixed-point tiles move
+# the same data but Bluestein lengths are powers of two more often.)
 NCU_DRAM_BYTES_PER_POINT = {"uneven_float": 2.708141e9 / 37465227,
                             "uneven_double": 5.925791e9 / 37465227}
-NCU_DRAM_BYTES_PER_LAUNCH = {"c2c_f32_4096x4096": 217.3e6, "c2c_f32_2p18x64": 216.7e6,
-                             "c2c_f32_2p20x16": 215.7e6, "c2c_f32_2p24": 215.9e6,
+NCU_DRAM_BYTES_PER_LAUNCH = {"c2c_f32_4096x4096": 213.2e6, "c2c_f32_2p18x64": 213.6e6,
+                             "c2c_f32_2p20x16": 215.7e6, "c2c_f32_2p24": 213.0e6,
                              "c2c4096": 18.7e6}
 
 
@@ -957,9 +959,9 @@ def dominant_kernel_roofline(wl, ms_step, lib, peak, peak_kind, launches_per_ste
         achieved = per_launch / (dur / 1e3) / 1e9
         per_transform = wl.algorithmic_bytes_per_step() / (ms_step / 1e3) / 1e9
         traffic = NCU_DRAM_BYTES_PER_LAUNCH.get(workload)
-        generic = wl.precision == "double" or getattr(wl, "tc", False)
-        kernel = ("k_pass_reg (one launch per pass)" if generic else
-                  "k_pass_bulk / k_pass_pipe / k_pass_pipe_wide (one launch per pass)")
+        kernel = ("k_fx_spec / k_pass_fx (one launch per pass)" if wl.precision == "double" else
+                  "k_pass_reg (one launch per pass)" if getattr(wl, "tc", False) else
+                  "k_pass_bulk / k_pass_async (one launch per pass)")
         return {"bound": "hbm", "achieved": round(achieved, 1), "peak": peak, "unit": "GB/s",
                 "frac": round(achieved / peak, 4), "traffic": traffic, "peak_source": peak_kind,
                 "kernel": kernel,
