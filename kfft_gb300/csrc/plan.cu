@@ -607,7 +607,14 @@ static PassDesc make_desc(const FftPlan& P, size_t pi, const vec2_t* in, const L
         d.load_mode = MODE_LANE;
         d.store_mode = MODE_LANE;
     } else if (d.lanes_j == 1) {
-        const uint32_t target = ((sizeof(vec2_t) == 8) ? 4096 : 2048) / std::max<uint32_t>(1, P.var.single_div);
+        // FP32: full tiles.  Double build: smaller ones, whose CTAs wait on fewer
+        // warps (2^24 points forward, us, tiles of 2048 points against 1024:
+        // length 128 207, 190; 256 215, 201; 512 213, 204; run-time tiles 100 342,
+        // 334; 210 429, 378; but 30 302, 306; 500 421, 434; 720 446, 454)
+        const bool pow2 = (s.R & (s.R - 1)) == 0;
+        const uint32_t full = sizeof(vec2_t) == 8 ? 4096
+                              : (pow2 || (s.R >= 64 && s.R < 256)) ? 1024 : 2048;
+        const uint32_t target = full / std::max<uint32_t>(1, P.var.single_div);
         C = std::max<uint32_t>(1, std::min(target / std::max<uint32_t>(s.R, 1), cap / std::max<uint32_t>(s.R, 1)));
         C = std::min(C, d.batch);
         d.load_mode = MODE_ELEM;
