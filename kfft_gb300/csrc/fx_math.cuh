@@ -91,6 +91,21 @@ __host__ __device__ constexpr int32_t fx_hi(fx_t v) {
     return int32_t((v - fx_t(l)) >> 32);
 }
 
+// cos or sin of 2 pi m / P as N + F / 2^64
+constexpr fx_t fx_const62(long m, long P, bool want_sin) {
+    m %= P;
+    if (m < 0) m += P;
+    const FxCosSin p = fx_cossin(uint64_t(m), uint64_t(P));
+    const fx_t v = want_sin ? p.s : p.c, h = kFxOne / 2;
+    // the halves, exactly
+    if (v - h > -64 && v - h < 64) return h;
+    if (v + h > -64 && v + h < 64) return -h;
+    return v;
+}
+// v = N + F / 2^64 with F in [-2^63, 2^63)
+constexpr int fx_const_n(fx_t v) { return v >= kFxOne / 2 ? 1 : (v < -(kFxOne / 2) ? -1 : 0); }
+constexpr fx_t fx_const_f(fx_t v) { return (v - fx_t(fx_const_n(v)) * kFxOne) * 4; }
+
 #if defined(__CUDACC__)
 // ---------------------------------------------------------------------------
 // products
@@ -201,21 +216,6 @@ __device__ __forceinline__ fx_t fx_mulc(fx_t x, FxLimbs l, int32_t one, fx_t acc
 // ---------------------------------------------------------------------------
 __device__ __forceinline__ cfx_t fx_add(cfx_t a, cfx_t b) { return {a.x + b.x, a.y + b.y}; }
 __device__ __forceinline__ cfx_t fx_sub(cfx_t a, cfx_t b) { return {a.x - b.x, a.y - b.y}; }
-
-// cos or sin of 2 pi m / P as N + F / 2^64
-constexpr fx_t fx_const62(long m, long P, bool want_sin) {
-    m %= P;
-    if (m < 0) m += P;
-    const FxCosSin p = fx_cossin(uint64_t(m), uint64_t(P));
-    const fx_t v = want_sin ? p.s : p.c, h = kFxOne / 2;
-    // the halves, exactly
-    if (v - h > -64 && v - h < 64) return h;
-    if (v + h > -64 && v + h < 64) return -h;
-    return v;
-}
-// v = N + F / 2^64 with F in [-2^63, 2^63)
-constexpr int fx_const_n(fx_t v) { return v >= kFxOne / 2 ? 1 : (v < -(kFxOne / 2) ? -1 : 0); }
-constexpr fx_t fx_const_f(fx_t v) { return (v - fx_t(fx_const_n(v)) * kFxOne) * 4; }
 
 // a * W_P^E (W = exp(-2 pi i / P)), E modulo P
 template <int P, int E>

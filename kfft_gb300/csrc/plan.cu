@@ -40,9 +40,10 @@ constexpr uint32_t kMultiLanes = 4;   // 64-byte row segments
 #endif
 
 // Multi-lane tiles of passes of 256 points or more hold half a full tile in
-// the FP64 build (measured faster there); FP32 tiles are full (with lanes
-// skewed in shared memory, a full tile of a 256-point pass measured 18-23%
-// faster than half of one).
+// the double build (64 x 2^18 forward 476 us, 490 with full ones; 512 x 2^15 475
+// against 464; passes below 256 points are slower with half tiles: 256 x 59049
+// 888 against 789); FP32 tiles are full (with lanes skewed in shared memory, a
+// full tile of a 256-point pass measured 18-23% faster than half of one).
 static uint32_t lane_share(uint32_t R) {
 #if defined(KFFT_HALF_SCALAR)
     (void)R;
