@@ -759,9 +759,41 @@ __device__ __forceinline__ void fused_load(const PassDesc& d, uint32_t bs, uint3
 // around, so those keep the first form.)
 enum : int { STORE_ANY = 0, STORE_PLAIN = 1, STORE_PRODUCT = 2 };
 
+#if defined(KFFT_HALF_SCALAR)
+// P outputs that lie side by side, 16 bytes a store: each thread fills whole
+// sectors of its own, and 8 bytes a store left the pass bound by the requests
+// (1400 tiles of 4096 points: 16-point sequences 49.4 -> 31.0 us, 12 points 47.2
+// -> 30.3, 10 points 37.5 -> 26.9).  Rows of odd length start on a 16-byte
+// boundary every second time: the element left over is the first or the last.
+template <int P>
+__device__ __forceinline__ bool store_row(vec2_t* o, const vec2_t* v, real_t scale) {
+    const bool off = (reinterpret_cast<uintptr_t>(o) & 15u) != 0;
+    if constexpr (P % 2 == 0) {
+        if (off) return false;
+        float4* w = reinterpret_cast<float4*>(o);
+#pragma unroll
+        for (int q = 0; q < P; q += 2) {
+            const vec2_t a = cscale(v[q], scale), b = cscale(v[q + 1], scale);
+            w[q / 2] = make_float4(a.x, a.y, b.x, b.y);
+        }
+    } else {
+        o[off ? 0 : P - 1] = cscale(off ? v[0] : v[P - 1], scale);
+        float4* w = reinterpret_cast<float4*>(off ? o + 1 : o);
+#pragma unroll
+        for (int q = 0; q + 1 < P; q += 2) {
+            const vec2_t a = cscale(off ? v[q + 1] : v[q], scale);
+            const vec2_t b = cscale(off ? v[q + 2] : v[q + 1], scale);
+            w[q / 2] = make_float4(a.x, a.y, b.x, b.y);
+        }
+    }
+    return true;
+}
+#endif
+
 // Stores the P outputs of one butterfly of the last inner pass straight to
-// global memory through the epilogue.
-template <int P, int STORE = STORE_ANY>
+// global memory through the epilogue.  UNIT: ns == 1, a pass of one stage, whose
+// plain stores may lie side by side (store_row).
+template <int P, int STORE = STORE_ANY, bool UNIT = false>
 __device__ __forceinline__ void fused_store(const PassDesc& d, uint32_t bs, uint32_t j, uint32_t ob,
                                             uint32_t ns, const vec2_t* v) {
     const uint32_t blo = fdiv(j, d.div_Ns);
@@ -770,6 +802,11 @@ __device__ __forceinline__ void fused_store(const PassDesc& d, uint32_t bs, uint
     if (STORE == STORE_PLAIN || (STORE == STORE_ANY && d.epi_op == EPI_NONE)) {
         vec2_t* o = d.out + uint64_t(bs) * d.out_bs + uint64_t(base + ob * d.Ns) * d.out_es;
         const uint64_t step = uint64_t(ns * d.Ns) * d.out_es;
+#if defined(KFFT_HALF_SCALAR)
+        if constexpr (UNIT) {
+            if (step == 1 && store_row<P>(o, v, d.scale)) return;
+        }
+#endif
 #pragma unroll
         for (int q = 0; q < P; ++q) o[q * step] = cscale(v[q], d.scale);
     } else if (STORE == STORE_PRODUCT && d.epi_op == EPI_RADER_INV) {
@@ -923,7 +960,8 @@ __device__ __forceinline__ void fused_pass(const PassDesc& d, const InnerStep& s
 #pragma unroll
             for (int q = 0; q < P; ++q) dst[c * d.lane_stride + slot<LIN>(ob + q * ns)] = v[q];
         } else if (live) {
-            fused_store<P, STORE>(d, bs, j, ob, ns, v);
+            if (STORE == STORE_PLAIN && ns == 1) fused_store<P, STORE, STORE == STORE_PLAIN>(d, bs, j, ob, 1, v);
+            else fused_store<P, STORE>(d, bs, j, ob, ns, v);
         }
     }
 }
@@ -1211,7 +1249,7 @@ __device__ __forceinline__ void spec_stage(const PassDesc& d, const vec2_t* __re
                 for (int q = 0; q < P; ++q) l0[pad(ob + q * NS)] = v[q];
             }
         } else if (live) {
-            fused_store<P, STORE>(d, bs, j, ob, NS, v);
+            fused_store<P, STORE, (NS == 1)>(d, bs, j, ob, NS, v);
         }
     }
 }
@@ -1317,7 +1355,7 @@ __device__ __forceinline__ void tile_loop_pipelined(const PassDesc& d, vec2_t* s
             dft<16, INV>(v);
             const uint32_t ob = jj0 * 16;
             if constexpr (NP == 1) {
-                if (live) fused_store<16>(d, bs, j, ob, 1, v);
+                if (live) fused_store<16, STORE_ANY, true>(d, bs, j, ob, 1, v);
             } else {
                 if constexpr (kPadShift >= 4) {
                     vec2_t* p0 = bufA + c0 * lstride + pad(ob);  // 16 slots inside one pad period
@@ -1446,7 +1484,7 @@ __device__ __forceinline__ void tile_loop_async(const PassDesc& d, bool pairs, v
         dft<16, INV>(v);
         const uint32_t ob = jj0 * 16;
         if constexpr (NP == 1) {
-            if (live) fused_store<16, STORE>(d, bs, j, ob, 1, v);
+            if (live) fused_store<16, STORE, true>(d, bs, j, ob, 1, v);
         } else {
             vec2_t* p0 = buf + c0 * lstride + pad(ob);  // 16 slots inside one pad period
 #pragma unroll
@@ -1585,7 +1623,7 @@ __device__ __forceinline__ void tile_loop_bulk(const PassDesc& d, unsigned char*
             dft<16, INV>(v);
             const uint32_t ob = jj0 * 16;
             if constexpr (NP == 1) {
-                if (live) fused_store<16, STORE>(d, g, 0, ob, 1, v);
+                if (live) fused_store<16, STORE, true>(d, g, 0, ob, 1, v);
             } else {
                 vec2_t* p0 = bufA + c0 * lstride + pad(ob);  // 16 slots inside one pad period
 #pragma unroll

@@ -89,3 +89,24 @@ def test_run_time_tiles_convolve(libf, y, x):
     assert rel_l2(got, ref * (1 if y % 2 else 2)) <= TOL32
     c = libf.conv2_cpx(a.astype(np.complex64), b.astype(np.complex64))
     assert rel_l2(c, ref) <= TOL32
+
+
+# one-stage batches: rows stored 16 bytes at a time, of even and odd length,
+# from an aligned address and from 8 bytes past one, and in place
+@pytest.mark.parametrize("off", [0, 1])
+@pytest.mark.parametrize("n", range(2, 17))
+def test_one_stage_rows(libf, n, off):
+    for batch in (1, 2 * 4096 // n + 3):
+        rng = np.random.default_rng(n)
+        x = (rng.standard_normal((batch, n), np.float32) + 1j * rng.standard_normal((batch, n), np.float32)).astype(np.complex64)
+        tx, px = device(x, off)
+        ty, py = device(np.full((batch + 1, n), 7, np.complex64), off)
+        ref = np.fft.fft(x.astype(np.complex128), axis=1)
+        p = libf._plan("kfft_config_cpx", n, 0)
+        assert libf.L.kfft_eval_cpx_batch(p, px, py, batch) == 0, libf.last_error()
+        y = ty[off:].cpu().numpy().reshape(batch + 1, n)
+        assert rel_l2(y[:batch], ref) <= TOL32
+        assert (y[batch] == 7).all()
+        assert libf.L.kfft_eval_cpx_batch(p, px, px, batch) == 0, libf.last_error()
+        libf.cleanup(p)
+        assert rel_l2(tx[off:].cpu().numpy().reshape(batch, n), ref) <= TOL32
