@@ -61,8 +61,11 @@ struct alignas(16) FxTw {
 constexpr uint32_t kFxLaneBytes = 32;
 // butterflies of radix P a thread of a run-time tile runs side by side
 constexpr uint32_t fx_group(uint32_t P) { return P == 2 ? 4 : (P == 3 ? 3 : (P <= 6 ? 2 : 1)); }
-// rows of lane words a fixed-point tile has at least (one a stage)
+// rows of lane words a fixed-point tile has at least (one a stage), and how many
+// more behind them: two (fx_guard_row) and, for a compile-time tile of R points
+// a lane, a bit an element
 constexpr uint32_t kFxRows = 4;
+constexpr uint32_t fx_guard_rows(uint32_t spec_R) { return 2 + (spec_R + 31) / 32; }
 // threads of a full power-of-two fixed-point tile (8 points each)
 constexpr uint32_t kFxSpecThreads = 512;
 // most threads of a run-time fixed-point tile

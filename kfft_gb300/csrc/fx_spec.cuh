@@ -125,7 +125,7 @@ __device__ __forceinline__ void fx_spec_later(const PassDesc& d, cfx_t* buf, uin
     const bool lane_mode = kLast && d.store_mode == MODE_LANE;
     uint32_t c[G], jj[G];
     cfx_t v[G][P];
-    __syncthreads();
+    if constexpr (IDX > 1) __syncthreads();  // (behind the first stage the tile has one)
 #pragma unroll
     for (int g = 0; g < G; ++g) {
         // threads past the last butterfly repeat it without storing
@@ -178,6 +178,46 @@ __device__ __forceinline__ void fx_spec_later(const PassDesc& d, cfx_t* buf, uin
     }
 }
 
+// The closer look at a tile with a lane that may need the FP64 body (fx_apart):
+// its elements read again.  Behind the rows of words one for what each lane
+// holds and a bit an element that is near its lane's largest.
+template <uint32_t R>
+__device__ __forceinline__ bool fx_spec_apart(const PassDesc& d, uint32_t* words, uint32_t lane0,
+                                              uint32_t total) {
+    constexpr uint32_t kBits = (R + 31) / 32;
+    uint32_t* holds = words + (kFxRows + 1) * d.C;
+    uint32_t* big = holds + d.C;
+    const bool lane_mode = d.load_mode == MODE_LANE;
+#pragma unroll 1
+    for (uint32_t i = threadIdx.x; i < d.C * R; i += blockDim.x) {
+        const uint32_t r = lane_mode ? fdiv(i, d.div_C) : i % R;
+        const uint32_t c = lane_mode ? i - r * d.C : i / R;
+        if (lane0 + c >= total || words[c] == 0) continue;
+        uint32_t b, j;
+        fx_lane(d, lane0 + c, b, j);
+        uint32_t n = j + r * d.lanes_j;
+        if (d.pro_op == PRO_GATHER) n = __ldg(&d.pro_perm[n]);
+        const double2 x = __ldcg(&d.in[uint64_t(b) * d.in_bs + uint64_t(n) * d.in_es]);
+        const uint32_t near = fx_near(words[c], fx_span(R, fx_spec_radix(R, 1)));
+        const uint32_t f = fx_holds(x, near);
+        if (f) atomicOr(&holds[c], f);
+        if (max(fx_mag(x.x), fx_mag(x.y)) >= near) atomicOr(&big[c * kBits + r / 32], 1u << (r % 32));
+    }
+    __syncthreads();
+    bool apart = false;
+    for (uint32_t c = threadIdx.x; c < d.C; c += blockDim.x) {
+        uint32_t f = holds[c];
+        const uint32_t* w = big + c * kBits;
+        for (uint32_t k = 0; k < kBits && fx_apart(f); ++k) {
+            // bit r with bit r + 1 (the first one behind the last)
+            const uint32_t up = w[k + 1 < kBits ? k + 1 : 0] & 1u;
+            if (w[k] & ((w[k] >> 1) | up << (R < 32 ? R - 1 : 31))) f |= FX_PAIR;
+        }
+        apart = apart || fx_apart(f);
+    }
+    return __syncthreads_or(apart);
+}
+
 // One tile (C * R <= 8 points a thread); false (with nothing written) when it
 // is one for the FP64 body.
 template <uint32_t R>
@@ -190,7 +230,8 @@ __device__ __forceinline__ bool fx_spec_tile(const PassDesc& d, uint32_t tile, u
     const uint32_t items = d.C * M;
     cfx_t* buf = reinterpret_cast<cfx_t*>(smem);
     uint32_t* words = reinterpret_cast<uint32_t*>(smem + d.fx_words);
-    for (uint32_t i = threadIdx.x; i < kFxRows * d.C; i += blockDim.x) words[i] = 0;
+    uint32_t* both = words + kFxRows * d.C;  // (fx_guard_row: at most four stages)
+    for (uint32_t i = threadIdx.x; i < (kFxRows + fx_guard_rows(R)) * d.C; i += blockDim.x) words[i] = 0;
     const bool lane_mode = d.load_mode == MODE_LANE;
     uint32_t c[G], jj[G];
     double2 raw[G][P];
@@ -232,13 +273,15 @@ __device__ __forceinline__ bool fx_spec_tile(const PassDesc& d, uint32_t tile, u
     for (int g = 0; g < G; ++g) {
         // the largest magnitude word: of the negative values (the unsigned
         // maximum) and of the others (the signed one)
-        uint32_t neg = 0, low = 0;
+        uint32_t neg = 0, low = 0, m2 = 0;
         int pos = 0;
 #pragma unroll
         for (int q = 0; q < P; ++q) {
             const int x = __double2hiint(raw[g][q].x), y = __double2hiint(raw[g][q].y);
             neg = __vimax3_u32(neg, uint32_t(x), uint32_t(y));
             pos = __vimax3_s32(pos, x, y);
+            // (two elements of each butterfly show nearly every lane that stays)
+            if (q == 0 || q == P / 2) m2 = max(m2, min(uint32_t(x) & 0x7fffffffu, uint32_t(y) & 0x7fffffffu));
             low |= uint32_t(__double2loint(raw[g][q].x)) | uint32_t(__double2loint(raw[g][q].y));
         }
         uint32_t m = max(neg & 0x7fffffffu, uint32_t(pos));
@@ -246,17 +289,23 @@ __device__ __forceinline__ bool fx_spec_tile(const PassDesc& d, uint32_t tile, u
         bad = bad || (m >> 20) >= kFxExpHigh || (m != 0 && (m >> 20) < kFxExpLow);
         if (M % 32 == 0 && !lane_mode) {
             m = __reduce_max_sync(0xffffffffu, m);
+            m2 = __reduce_max_sync(0xffffffffu, m2);
             if ((threadIdx.x & 31) == 0 && m) atomicMax(&words[c[g]], m);
+            if ((threadIdx.x & 31) == 0 && m2) atomicMax(&both[c[g]], m2);
         } else {
             atomicMax(&words[c[g]], m);
+            atomicMax(&both[c[g]], m2);
         }
     }
     if (__syncthreads_or(bad)) return false;
     const bool outer = d.Ns > 1, chirp = d.pro_op == PRO_CHIRP, inv = d.inv != 0;
     const int top = (outer || chirp ? 61 : 59) - fx_room(P);
+    bool rare = false;
     cfx_t v[G][P];
 #pragma unroll
     for (int g = 0; g < G; ++g) {
+        // (a chirp turns every element, so nothing stays apart)
+        rare = rare || (!chirp && words[c[g]] != 0 && both[c[g]] < fx_near(words[c[g]], fx_span(R, P)));
         {
             const int field = int(words[c[g]] >> 20);
             const int emax = field ? field : 4096;  // a lane of zeros: everything shifts out
@@ -290,6 +339,7 @@ __device__ __forceinline__ bool fx_spec_tile(const PassDesc& d, uint32_t tile, u
         }
     }
     fx_spec_exchange<P, G, R, 1>(d, buf, words + d.C, c, jj, v, lane_mode);
+    if (__syncthreads_or(rare) && fx_spec_apart<R>(d, words, lane0, total)) return false;
     fx_spec_later<R, P, 1>(d, buf, words, lane0, total);
     return true;
 }

@@ -26,7 +26,11 @@
 // uneven batch of 256 in 1672 us, they run it in 887.
 //
 // A tile that holds an infinity, a NaN or magnitudes outside 2^-767 .. 2^767
-// is left to the FP64 body, which treats them as IEEE arithmetic does.
+// is left to the FP64 body, which treats them as IEEE arithmetic does, and so
+// is one with a lane whose small parts doubles would keep apart from its large
+// ones (fx_apart in fx_math.cuh).  Telling the lanes costs 1 to 2% (4096 x 256
+// both ways 51.4 -> 51.7 us, uneven batch of 256 826 -> 841); real values in
+// the complex form take the closer look (4096 x 1024 points 70.6 -> 91.6).
 #pragma once
 
 #include "fft_device.cuh"
@@ -85,6 +89,18 @@ struct __align__(16) FxLane {
 };
 static_assert(sizeof(FxLane) == kFxLaneBytes, "the planner sizes shared memory with it");
 constexpr uint32_t kFxDead = 0xffffffffu;
+
+// magnitude word of a part
+__device__ __forceinline__ uint32_t fx_mag(double v) { return uint32_t(__double2hiint(v)) & 0x7fffffffu; }
+
+__device__ __forceinline__ uint32_t fx_holds(double2 x, uint32_t near) {
+    return fx_holds(fx_mag(x.x), fx_mag(x.y), x.x != 0.0, x.y != 0.0, near);
+}
+
+// first of the two rows of words behind the stages' ones: the largest of the
+// elements' smaller parts (a lane where it is near the largest stays without a
+// closer look), and what the lane holds (FX_HAS_RE ...)
+__device__ __forceinline__ uint32_t fx_guard_row(const PassDesc& d) { return max(uint32_t(d.nrad), kFxRows); }
 
 // sequence and lane index of lane g of a pass
 __device__ __forceinline__ void fx_lane(const PassDesc& d, uint32_t g, uint32_t& b, uint32_t& j) {
@@ -162,10 +178,16 @@ __device__ __forceinline__ bool fx_read(const PassDesc& d, cfx_t* buf, uint32_t*
     const uint64_t step = uint64_t(d.lanes_j) * d.in_es;
     constexpr int U = 4;  // loads in flight together
     uint32_t any = 0, small = 0xffffffffu;
+    uint32_t* both = words + fx_guard_row(d) * d.C;
     {
-        // the raw doubles to shared memory, the largest of each lane to words
+        // the raw doubles to shared memory, the largest of each lane to words,
+        // the largest of the smaller parts to both
         FxWalk w(d, lane_mode);
-        uint32_t seen = w.c, most = 0;
+        uint32_t seen = w.c, most = 0, most2 = 0;
+        auto flush = [&] {
+            if (most) atomicMax(&words[seen], most);
+            if (most2) atomicMax(&both[seen], most2);
+        };
 #pragma unroll 1
         for (uint32_t i = threadIdx.x; i < elems; i += U * blockDim.x) {
             double2 v[U];
@@ -191,27 +213,50 @@ __device__ __forceinline__ bool fx_read(const PassDesc& d, cfx_t* buf, uint32_t*
             for (int u = 0; u < U; ++u) {
                 if (i + u * blockDim.x >= elems) break;
                 reinterpret_cast<double2*>(buf)[at[u]] = v[u];
-                uint32_t m = max(uint32_t(__double2hiint(v[u].x)) & 0x7fffffffu,
-                                 uint32_t(__double2hiint(v[u].y)) & 0x7fffffffu);
+                const uint32_t a = fx_mag(v[u].x), b = fx_mag(v[u].y);
+                uint32_t m = max(a, b);
                 if (m == 0 && (__double2loint(v[u].x) | __double2loint(v[u].y))) m = 1;
                 any = max(any, m);
                 if (m) small = min(small, m);
                 if (c[u] != seen) {
-                    if (most) atomicMax(&words[seen], most);
+                    flush();
                     seen = c[u];
-                    most = 0;
+                    most = most2 = 0;
                 }
                 most = max(most, m);
+                most2 = max(most2, min(a, b));
             }
         }
         if (d.C == 1) {
             most = __reduce_max_sync(0xffffffffu, most);
-            if ((threadIdx.x & 31) == 0 && most) atomicMax(&words[0], most);
-        } else if (most) {
-            atomicMax(&words[seen], most);
+            most2 = __reduce_max_sync(0xffffffffu, most2);
         }
+        if (d.C > 1 || (threadIdx.x & 31) == 0) flush();
     }
     if (__syncthreads_or((any >> 20) >= kFxExpHigh || (small >> 20) < kFxExpLow)) return false;
+    // (a chirp turns every element, so nothing stays apart)
+    const int span = fx_span(d.R, d.rad[0]);
+    bool rare = false;
+    if (d.pro_op != PRO_CHIRP)
+        for (uint32_t c = threadIdx.x; c < d.C; c += blockDim.x)
+            rare = rare || (words[c] != 0 && both[c] < fx_near(words[c], span));
+    if (__syncthreads_or(rare)) {
+        uint32_t* holds = both + d.C;
+        FxWalk w(d, false);
+#pragma unroll 1
+        for (uint32_t i = threadIdx.x; i < elems; i += blockDim.x, w.next(d)) {
+            const double2* lane = reinterpret_cast<const double2*>(&buf[w.c * d.lane_stride]);
+            const uint32_t near = fx_near(words[w.c], span), r1 = w.r + 1 == d.R ? 0 : w.r + 1;
+            const double2 x = lane[pad(w.r)], y = lane[pad(r1)];
+            uint32_t f = fx_holds(x, near);
+            if (max(fx_mag(x.x), fx_mag(x.y)) >= near && max(fx_mag(y.x), fx_mag(y.y)) >= near) f |= FX_PAIR;
+            if (f) atomicOr(&holds[w.c], f);
+        }
+        __syncthreads();
+        bool apart = false;
+        for (uint32_t c = threadIdx.x; c < d.C; c += blockDim.x) apart = apart || fx_apart(holds[c]);
+        if (__syncthreads_or(apart)) return false;
+    }
     // each thread its own elements again: integers against their lane's scale
     const bool outer = d.Ns > 1, chirp = d.pro_op == PRO_CHIRP, inv = d.inv != 0;
     const int top = (outer || chirp ? 61 : 59) - fx_room(d.rad[0]);
@@ -381,7 +426,7 @@ __device__ __forceinline__ bool fx_tile(const PassDesc& d, const PassExtra& x, u
     cfx_t* bufB = d.inplace ? bufA : bufA + d.C * d.lane_stride + 1;
     uint32_t* words = reinterpret_cast<uint32_t*>(smem + d.fx_words);
     FxLane* lanes = reinterpret_cast<FxLane*>(smem + d.fx_lanes);
-    for (uint32_t i = threadIdx.x; i < d.nrad * d.C; i += blockDim.x) words[i] = 0;
+    for (uint32_t i = threadIdx.x; i < (fx_guard_row(d) + 2) * d.C; i += blockDim.x) words[i] = 0;
     fx_lanes(d, lanes, tile * d.C, d.batch * d.lanes_j);
     __syncthreads();
     if (!fx_read(d, bufA, words, lanes)) return false;

@@ -45,6 +45,16 @@ __global__ void __launch_bounds__(T, BLOCKS) k_pass_fx(const __grid_constant__ P
     double_tile(d, x, blockIdx.x, smem_raw);
 }
 
+// Passes of 2 and 4 points: in doubles, one butterfly a thread, straight from
+// global memory to global memory.
+template <bool INV>
+__global__ void __launch_bounds__(kFxWideThreads) k_pass_short(const __grid_constant__ PassDesc d,
+                                                             const __grid_constant__ PassExtra x) {
+    const uint32_t lane0 = blockIdx.x * d.C, total = d.batch * d.lanes_j;
+    if (d.R == 2) fused_pass<2, INV, STORE_ANY, false>(d, x.step[0], nullptr, nullptr, lane0, total, IO_GLOBAL, IO_GLOBAL);
+    else fused_pass<4, INV, STORE_ANY, false>(d, x.step[0], nullptr, nullptr, lane0, total, IO_GLOBAL, IO_GLOBAL);
+}
+
 FxKernel fx_kernels_1(uint32_t spec);
 FxKernel fx_kernels_2(uint32_t spec);
 FxKernel fx_kernels_3(uint32_t spec);
@@ -80,7 +90,12 @@ void launch_pass_reg(const PassDesc& d, const PassExtra& x, cudaStream_t st) {
         note_cuda_error(k.error);
         return;
     }
-    k.f[d.fx && d.spec ? d.spec : (d.threads > kPassThreads ? 1 : 0)]<<<d.tiles, d.threads, d.smem_bytes, st>>>(d, x);
+    if (!d.fx && d.nrad == 1) {
+        if (d.inv) k_pass_short<true><<<d.tiles, d.threads, 0, st>>>(d, x);
+        else k_pass_short<false><<<d.tiles, d.threads, 0, st>>>(d, x);
+    } else {
+        k.f[d.spec ? d.spec : (d.threads > kPassThreads ? 1 : 0)]<<<d.tiles, d.threads, d.smem_bytes, st>>>(d, x);
+    }
     note_cuda_error(cudaGetLastError());
     count_launch();
 }
