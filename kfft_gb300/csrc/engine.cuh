@@ -86,7 +86,7 @@ enum : uint8_t {
     EPI_MUL = 1,       // out[b*bs + k*es] = v * tab[k]
     EPI_CHIRP = 2,     // k < bound: out[b*bs + k*es] = v * tab[k] * scale
     EPI_RADER_FWD = 3, // out[..k..] = v * tab[k]; k == 0: aux_out[2b] = x0, aux_out[2b+1] = x0 + v
-    EPI_RADER_INV = 4, // aux_out[b*bs + perm[k]*es] = (v + x0) * scale; k == 0 also X_0
+    EPI_RADER_INV = 4, // aux_out[b*bs + perm[k]*es] = (v + aux_in[2b]) * scale; k == 0 also X_0
     EPI_MUL_OUT = 5,   // out[i] = v * tab[i] * scale, i = b*bs + k*es: a table in the output's
                        // layout (the other operand's spectrum of a convolution)
 };

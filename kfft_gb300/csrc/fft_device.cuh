@@ -484,15 +484,15 @@ __device__ __forceinline__ void store_elem(const PassDesc& d, uint32_t b, uint32
             break;
         case EPI_RADER_FWD:
             // spectrum of the gathered sequence times the kernel spectrum; bin 0
-            // is sum_{n>=1} x_n, so X_0 = x_0 + v is saved per sequence, and x_0
-            // added to bin 0 of the product adds x_0 to every output of the
-            // (unnormalised) inverse
+            // is sum_{n>=1} x_n, so X_0 = x_0 + v is saved with x_0 per sequence.
+            // (x_0 in bin 0 of the product would add it to every output too, but
+            // through the inverse's twiddles: an infinite one would leave NaN in
+            // the part it does not touch, and a large one its rounding in both.)
+            d.out[b * d.out_bs + uint64_t(k) * d.out_es] = cmul(v, __ldg(&d.epi_tab[k]));
             if (k == 0) {
                 const vec2_t x0 = __ldcg(&d.aux_in[b * d.aux_in_bs]);
-                d.aux_out[b] = cadd(x0, v);
-                d.out[b * d.out_bs] = cadd(cmul(v, __ldg(&d.epi_tab[0])), x0);
-            } else {
-                d.out[b * d.out_bs + uint64_t(k) * d.out_es] = cmul(v, __ldg(&d.epi_tab[k]));
+                d.aux_out[2 * uint64_t(b)] = x0;
+                d.aux_out[2 * uint64_t(b) + 1] = cadd(x0, v);
             }
             break;
         case EPI_MUL_OUT: {
@@ -501,12 +501,13 @@ __device__ __forceinline__ void store_elem(const PassDesc& d, uint32_t b, uint32
             break;
         }
         case EPI_RADER_INV: {
-            // X[g^-k] = v (x_0 is in it), and the saved X_0; never reads the input,
+            // X[g^-k] = x_0 + c_k, and X_0 from the saved pair; never reads the input,
             // so the transform may run in place
+            const vec2_t x0 = __ldcg(&d.aux_in[2 * uint64_t(b)]);
             const uint32_t idx = __ldg(&d.epi_perm[k]);
             vec2_t* o = d.aux_out + b * d.aux_out_bs;
-            o[uint64_t(idx) * d.aux_out_es] = cscale(v, d.scale);
-            if (k == 0) o[0] = cscale(__ldcg(&d.aux_in[b]), d.scale);
+            o[uint64_t(idx) * d.aux_out_es] = cscale(cadd(v, x0), d.scale);
+            if (k == 0) o[0] = cscale(__ldcg(&d.aux_in[2 * uint64_t(b) + 1]), d.scale);
             break;
         }
         default:
@@ -813,7 +814,8 @@ __device__ __forceinline__ void fused_store(const PassDesc& d, uint32_t bs, uint
         constexpr int G = P < 8 ? P : 8;
         const uint32_t k = base + ob * d.Ns, ks = ns * d.Ns;
         vec2_t* o = d.aux_out + uint64_t(bs) * d.aux_out_bs;
-        if (k == 0) o[0] = cscale(__ldcg(&d.aux_in[bs]), d.scale);
+        const vec2_t x0 = __ldcg(&d.aux_in[2 * uint64_t(bs)]);
+        if (k == 0) o[0] = cscale(__ldcg(&d.aux_in[2 * uint64_t(bs) + 1]), d.scale);
 #pragma unroll
         for (int g = 0; g < P; g += G) {
             uint32_t at[G];
@@ -822,7 +824,7 @@ __device__ __forceinline__ void fused_store(const PassDesc& d, uint32_t bs, uint
                 if (g + u < P) at[u] = __ldg(&d.epi_perm[k + (g + u) * ks]);
 #pragma unroll
             for (int u = 0; u < G; ++u)
-                if (g + u < P) o[uint64_t(at[u]) * d.aux_out_es] = cscale(v[g + u], d.scale);
+                if (g + u < P) o[uint64_t(at[u]) * d.aux_out_es] = cscale(cadd(v[g + u], x0), d.scale);
         }
     } else if (STORE == STORE_PRODUCT) {
         // (loading and storing one after the other took twice the time: 34 x
@@ -845,13 +847,12 @@ __device__ __forceinline__ void fused_store(const PassDesc& d, uint32_t bs, uint
 #pragma unroll
             for (int u = 0; u < G; ++u)
                 if (g + u < P && k + u * ks < bound) {
-                    vec2_t r = cscale(cmul(v[g + u], w[u]), scale);
                     if (g + u == 0 && rader && k == 0) {  // (as in store_elem)
                         const vec2_t x0 = __ldcg(&d.aux_in[uint64_t(bs) * d.aux_in_bs]);
-                        d.aux_out[bs] = cadd(x0, v[0]);
-                        r = cadd(r, x0);
+                        d.aux_out[2 * uint64_t(bs)] = x0;
+                        d.aux_out[2 * uint64_t(bs) + 1] = cadd(x0, v[0]);
                     }
-                    o[uint64_t(k + u * ks) * es] = r;
+                    o[uint64_t(k + u * ks) * es] = cscale(cmul(v[g + u], w[u]), scale);
                 }
             k += G * ks;
         }

@@ -42,7 +42,7 @@ __device__ __forceinline__ void fx_spec_store(const PassDesc& d, uint32_t g, uin
     const bool inv = d.inv != 0;
     const uint32_t op = d.epi_op;
     const bool table = op == EPI_MUL || op == EPI_CHIRP || op == EPI_RADER_FWD;
-    const bool scaled = op == EPI_NONE || op == EPI_CHIRP || op == EPI_RADER_INV;
+    const bool scaled = op == EPI_NONE || op == EPI_CHIRP;
     const int32_t sh = scaled ? d.fx_scale_h : 0, sl = d.fx_scale_l;
     const int e_out = eb + (scaled ? d.fx_scale_e : 0) + (sh ? 2 : 0) + (table ? 2 : 0) +
                       (table && op != EPI_CHIRP ? d.fx_epi_e : 0);
@@ -56,10 +56,7 @@ __device__ __forceinline__ void fx_spec_store(const PassDesc& d, uint32_t g, uin
         if (table) {
             if (op == EPI_CHIRP && k >= d.epi_bound) continue;
             if (op == EPI_RADER_FWD && k == 0) {
-                const double2 x0 = __ldcg(&d.aux_in[b * d.aux_in_bs]);
-                d.aux_out[b] = cadd(x0, double2{fx_to_double(u.x, eb), fx_to_double(u.y, eb)});
-                u = fx_cmul(u, fx_tw_load(d.fx_epi), d.fx_one);
-                out[0] = cadd(x0, double2{fx_to_double(u.x, e_out), fx_to_double(u.y, e_out)});
+                store_elem(d, b, 0, double2{fx_to_double(u.x, eb), fx_to_double(u.y, eb)});
                 continue;
             }
             u = fx_cmul(u, fx_tw_load(&d.fx_epi[k]), d.fx_one);
@@ -75,7 +72,9 @@ __device__ __forceinline__ void fx_spec_store(const PassDesc& d, uint32_t g, uin
         if (op == EPI_RADER_INV) {
             o = d.aux_out + uint64_t(b) * d.aux_out_bs;
             at = uint64_t(__ldg(&d.epi_perm[k])) * d.aux_out_es;
-            if (k == 0) o[0] = cscale(__ldcg(&d.aux_in[b]), d.scale);
+            r = cadd(r, d.aux_in[2 * uint64_t(b)]);
+            if ((d.fx_scale_h | d.fx_scale_e) != 0) r = cscale(r, d.scale);  // scale != 1
+            if (k == 0) o[0] = cscale(__ldcg(&d.aux_in[2 * uint64_t(b) + 1]), d.scale);
         } else if (op == EPI_MUL_OUT) {
             r = cscale(cmul(r, __ldcg(&d.epi_tab[uint64_t(b) * d.out_bs + at])), d.scale);
         }

@@ -370,7 +370,7 @@ __device__ __forceinline__ void fx_write(const PassDesc& d, const cfx_t* buf, co
     const uint32_t op = d.epi_op;
     const bool table = op == EPI_MUL || op == EPI_CHIRP || op == EPI_RADER_FWD;
     // the scale: a power of two, times a factor where it is not one
-    const bool scaled = op == EPI_NONE || op == EPI_CHIRP || op == EPI_RADER_INV;
+    const bool scaled = op == EPI_NONE || op == EPI_CHIRP;
     const int32_t sh = scaled ? d.fx_scale_h : 0, sl = d.fx_scale_l;
     const int e_more = (scaled ? d.fx_scale_e : 0) + (sh ? 2 : 0) + (table ? 2 : 0) +
                        (table && op != EPI_CHIRP ? d.fx_epi_e : 0);
@@ -389,12 +389,9 @@ __device__ __forceinline__ void fx_write(const PassDesc& d, const cfx_t* buf, co
         double2* out = d.out;
         if (table) {
             if (op == EPI_RADER_FWD && k == 0) {
-                // X_0 = x_0 + the sum of the others; x_0 in bin 0 of the product
-                // adds x_0 to every output of the convolution
-                const double2 x0 = __ldcg(&d.aux_in[l.b * d.aux_in_bs]);
-                d.aux_out[l.b] = cadd(x0, double2{fx_to_double(u.x, eb), fx_to_double(u.y, eb)});
-                u = fx_cmul(u, fx_tw_load(d.fx_epi), d.fx_one);
-                out[at] = cadd(x0, double2{fx_to_double(u.x, eb + e_more), fx_to_double(u.y, eb + e_more)});
+                // in doubles: bin 0 of the spectrum is far below the others, and
+                // X_0 = x_0 + the sum of the others is saved with x_0
+                store_elem(d, l.b, 0, double2{fx_to_double(u.x, eb), fx_to_double(u.y, eb)});
                 continue;
             }
             u = fx_cmul(u, fx_tw_load(&d.fx_epi[k]), d.fx_one);
@@ -408,7 +405,9 @@ __device__ __forceinline__ void fx_write(const PassDesc& d, const cfx_t* buf, co
         if (op == EPI_RADER_INV) {
             out = d.aux_out + uint64_t(l.b) * d.aux_out_bs;
             at = uint64_t(__ldg(&d.epi_perm[k])) * d.aux_out_es;
-            if (k == 0) out[0] = cscale(__ldcg(&d.aux_in[l.b]), d.scale);
+            r = cadd(r, d.aux_in[2 * uint64_t(l.b)]);  // (a cached load: one value a sequence)
+            if ((d.fx_scale_h | d.fx_scale_e) != 0) r = cscale(r, d.scale);  // scale != 1
+            if (k == 0) out[0] = cscale(__ldcg(&d.aux_in[2 * uint64_t(l.b) + 1]), d.scale);
         } else if (op == EPI_MUL_OUT) {
             r = cscale(cmul(r, __ldcg(&d.epi_tab[at])), d.scale);
         }

@@ -547,7 +547,7 @@ size_t workspace_bytes(const FftPlan& p, uint32_t batch) {
         return 0;
     }
     size_t a = round256(sizeof(vec2_t) * size_t(p.L) * batch);
-    size_t extra = (p.method == METHOD_RADER) ? round256(sizeof(vec2_t) * size_t(batch)) : 0;
+    size_t extra = (p.method == METHOD_RADER) ? round256(sizeof(vec2_t) * 2 * size_t(batch)) : 0;
     return a + extra + std::max(workspace_bytes(*p.sub_fwd, batch), workspace_bytes(*p.sub_inv, batch));
 }
 
@@ -865,8 +865,8 @@ bool build_passes(const FftPlan& P, const vec2_t* in, const Layout& lin, vec2_t*
         return build_direct_passes(*P.sub_inv, A, la, out, lout, scale, fi, ws, descs);
     }
     // Rader
-    vec2_t* sums = ws.take(size_t(B));  // X_0 of each sequence
-    if (!sums) return false;
+    vec2_t* pairs = ws.take(size_t(2) * B);  // x_0 and X_0 of each sequence
+    if (!pairs) return false;
     Fuse ff;
     ff.pro_op = PRO_GATHER;
     ff.pro_perm = P.gperm;
@@ -878,14 +878,14 @@ bool build_passes(const FftPlan& P, const vec2_t* in, const Layout& lin, vec2_t*
 #endif
     ff.aux_in = in;
     ff.aux_in_bs = lin.bs;
-    ff.aux_out = sums;
+    ff.aux_out = pairs;
     const size_t mark = ws.used;
     if (!build_direct_passes(*P.sub_fwd, in, lin, A, la, real_t(1), ff, ws, descs)) return false;
     ws.used = mark;  // the inverse reuses the forward's scratch (stream ordered)
     Fuse fi;
     fi.epi_op = EPI_RADER_INV;
     fi.epi_perm = P.iperm;
-    fi.aux_in = sums;
+    fi.aux_in = pairs;
     fi.aux_out = out;
     fi.aux_out_bs = lout.bs;
     fi.aux_out_es = lout.es;
