@@ -177,8 +177,8 @@ __device__ __forceinline__ void fx_spec_later(const PassDesc& d, cfx_t* buf, uin
     }
 }
 
-// The closer look at a tile with a lane that may need the FP64 body (fx_apart):
-// its elements read again.  Behind the rows of words one for what each lane
+// The closer look at a tile with a lane that may need the FP64 body (fx_tiny,
+// fx_apart): its elements read again.  Behind the rows of words one for what each lane
 // holds and a bit an element that is near its lane's largest.
 template <uint32_t R>
 __device__ __forceinline__ bool fx_spec_apart(const PassDesc& d, uint32_t* words, uint32_t lane0,
@@ -187,6 +187,9 @@ __device__ __forceinline__ bool fx_spec_apart(const PassDesc& d, uint32_t* words
     uint32_t* holds = words + (kFxRows + 1) * d.C;
     uint32_t* big = holds + d.C;
     const bool lane_mode = d.load_mode == MODE_LANE;
+    bool tiny = false;
+    for (uint32_t c = threadIdx.x; c < d.C; c += blockDim.x) tiny = tiny || fx_tiny(words[c]);
+    if (__syncthreads_or(tiny)) return true;
 #pragma unroll 1
     for (uint32_t i = threadIdx.x; i < d.C * R; i += blockDim.x) {
         const uint32_t r = lane_mode ? fdiv(i, d.div_C) : i % R;
@@ -285,7 +288,7 @@ __device__ __forceinline__ bool fx_spec_tile(const PassDesc& d, uint32_t tile, u
         }
         uint32_t m = max(neg & 0x7fffffffu, uint32_t(pos));
         if (m == 0 && low) m = 1;
-        bad = bad || (m >> 20) >= kFxExpHigh || (m != 0 && (m >> 20) < kFxExpLow);
+        bad = bad || (m >> 20) >= kFxExpHigh;
         if (M % 32 == 0 && !lane_mode) {
             m = __reduce_max_sync(0xffffffffu, m);
             m2 = __reduce_max_sync(0xffffffffu, m2);
@@ -304,7 +307,8 @@ __device__ __forceinline__ bool fx_spec_tile(const PassDesc& d, uint32_t tile, u
 #pragma unroll
     for (int g = 0; g < G; ++g) {
         // (a chirp turns every element, so nothing stays apart)
-        rare = rare || (!chirp && words[c[g]] != 0 && both[c[g]] < fx_near(words[c[g]], fx_span(R, P)));
+        rare = rare || fx_tiny(words[c[g]]) ||
+               (!chirp && words[c[g]] != 0 && both[c[g]] < fx_near(words[c[g]], fx_span(R, P)));
         {
             const int field = int(words[c[g]] >> 20);
             const int emax = field ? field : 4096;  // a lane of zeros: everything shifts out

@@ -25,9 +25,10 @@
 // 16384 x 1000 417 against 566.  The FP64 body these tiles replace ran the
 // uneven batch of 256 in 1672 us, they run it in 887.
 //
-// A tile that holds an infinity, a NaN or magnitudes outside 2^-767 .. 2^767
-// is left to the FP64 body, which treats them as IEEE arithmetic does, and so
-// is one with a lane whose small parts doubles would keep apart from its large
+// A tile that holds an infinity, a NaN, a magnitude from 2^768 on or a lane
+// whose largest is below 2^-767 is left to the FP64 body, which treats them as
+// IEEE arithmetic does (smaller values beside larger ones shift out), and so is
+// one with a lane whose small parts doubles would keep apart from its large
 // ones (fx_apart in fx_math.cuh).  Telling the lanes costs 1 to 2% (4096 x 256
 // both ways 51.4 -> 51.7 us, uneven batch of 256 826 -> 841); real values in
 // the complex form take the closer look (4096 x 1024 points 70.6 -> 91.6).
@@ -40,8 +41,10 @@
 
 namespace kfft {
 
-// exponent fields outside this range go to the FP64 body
+// a lane's largest exponent field outside this range goes to the FP64 body
 constexpr uint32_t kFxExpLow = 256, kFxExpHigh = 1791;
+__device__ __forceinline__ bool fx_tiny(uint32_t most) { return most != 0 && (most >> 20) < kFxExpLow; }
+
 __device__ __forceinline__ FxTw fx_tw_load(const FxTw* p) {
     const int4 v = __ldg(reinterpret_cast<const int4*>(p));
     return {v.x, v.y, v.z, v.w};
@@ -177,7 +180,7 @@ __device__ __forceinline__ bool fx_read(const PassDesc& d, cfx_t* buf, uint32_t*
     const bool lane_mode = d.load_mode == MODE_LANE;
     const uint64_t step = uint64_t(d.lanes_j) * d.in_es;
     constexpr int U = 4;  // loads in flight together
-    uint32_t any = 0, small = 0xffffffffu;
+    uint32_t any = 0;
     uint32_t* both = words + fx_guard_row(d) * d.C;
     {
         // the raw doubles to shared memory, the largest of each lane to words,
@@ -217,7 +220,6 @@ __device__ __forceinline__ bool fx_read(const PassDesc& d, cfx_t* buf, uint32_t*
                 uint32_t m = max(a, b);
                 if (m == 0 && (__double2loint(v[u].x) | __double2loint(v[u].y))) m = 1;
                 any = max(any, m);
-                if (m) small = min(small, m);
                 if (c[u] != seen) {
                     flush();
                     seen = c[u];
@@ -233,14 +235,17 @@ __device__ __forceinline__ bool fx_read(const PassDesc& d, cfx_t* buf, uint32_t*
         }
         if (d.C > 1 || (threadIdx.x & 31) == 0) flush();
     }
-    if (__syncthreads_or((any >> 20) >= kFxExpHigh || (small >> 20) < kFxExpLow)) return false;
+    if (__syncthreads_or((any >> 20) >= kFxExpHigh)) return false;
     // (a chirp turns every element, so nothing stays apart)
+    const bool chirped = d.pro_op == PRO_CHIRP;
     const int span = fx_span(d.R, d.rad[0]);
-    bool rare = false;
-    if (d.pro_op != PRO_CHIRP)
-        for (uint32_t c = threadIdx.x; c < d.C; c += blockDim.x)
-            rare = rare || (words[c] != 0 && both[c] < fx_near(words[c], span));
-    if (__syncthreads_or(rare)) {
+    bool rare = false, tiny = false;
+    for (uint32_t c = threadIdx.x; c < d.C; c += blockDim.x) {
+        tiny = tiny || fx_tiny(words[c]);
+        rare = rare || (!chirped && words[c] != 0 && both[c] < fx_near(words[c], span));
+    }
+    if (__syncthreads_or(rare || tiny)) {
+        if (__syncthreads_or(tiny)) return false;
         uint32_t* holds = both + d.C;
         FxWalk w(d, false);
 #pragma unroll 1
@@ -258,7 +263,7 @@ __device__ __forceinline__ bool fx_read(const PassDesc& d, cfx_t* buf, uint32_t*
         if (__syncthreads_or(apart)) return false;
     }
     // each thread its own elements again: integers against their lane's scale
-    const bool outer = d.Ns > 1, chirp = d.pro_op == PRO_CHIRP, inv = d.inv != 0;
+    const bool outer = d.Ns > 1, chirp = chirped, inv = d.inv != 0;
     const int top = (outer || chirp ? 61 : 59) - fx_room(d.rad[0]);
     FxWalk w(d, lane_mode);
 #pragma unroll 2
