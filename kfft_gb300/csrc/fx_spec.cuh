@@ -190,20 +190,36 @@ __device__ __forceinline__ bool fx_spec_apart(const PassDesc& d, uint32_t* words
     bool tiny = false;
     for (uint32_t c = threadIdx.x; c < d.C; c += blockDim.x) tiny = tiny || fx_tiny(words[c]);
     if (__syncthreads_or(tiny)) return true;
-#pragma unroll 1
+    // rows of 32 elements or more, element by element: a warp has one lane's and
+    // a word of bits (whole warps: C * R and the threads are multiples of 32)
+    const bool by_warp = R >= 32 && !lane_mode;
+#pragma unroll 4
     for (uint32_t i = threadIdx.x; i < d.C * R; i += blockDim.x) {
         const uint32_t r = lane_mode ? fdiv(i, d.div_C) : i % R;
         const uint32_t c = lane_mode ? i - r * d.C : i / R;
-        if (lane0 + c >= total || words[c] == 0) continue;
-        uint32_t b, j;
-        fx_lane(d, lane0 + c, b, j);
-        uint32_t n = j + r * d.lanes_j;
-        if (d.pro_op == PRO_GATHER) n = __ldg(&d.pro_perm[n]);
-        const double2 x = __ldcg(&d.in[uint64_t(b) * d.in_bs + uint64_t(n) * d.in_es]);
-        const uint32_t near = fx_near(words[c], fx_span(R, fx_spec_radix(R, 1)));
-        const uint32_t f = fx_holds(x, near);
-        if (f) atomicOr(&holds[c], f);
-        if (max(fx_mag(x.x), fx_mag(x.y)) >= near) atomicOr(&big[c * kBits + r / 32], 1u << (r % 32));
+        uint32_t f = 0;
+        bool near = false;
+        if (lane0 + c < total && words[c] != 0) {
+            uint32_t b, j;
+            fx_lane(d, lane0 + c, b, j);
+            uint32_t n = j + r * d.lanes_j;
+            if (d.pro_op == PRO_GATHER) n = __ldg(&d.pro_perm[n]);
+            const double2 x = __ldcg(&d.in[uint64_t(b) * d.in_bs + uint64_t(n) * d.in_es]);
+            const uint32_t from = fx_near(words[c], fx_span(R, fx_spec_radix(R, 1)));
+            f = fx_holds(x, from);
+            near = max(fx_mag(x.x), fx_mag(x.y)) >= from;
+        }
+        if (by_warp) {
+            f = __reduce_or_sync(0xffffffffu, f);
+            const uint32_t bits = __ballot_sync(0xffffffffu, near);
+            if ((threadIdx.x & 31) == 0) {
+                if (f) atomicOr(&holds[c], f);
+                big[c * kBits + r / 32] = bits;
+            }
+        } else {
+            if (f) atomicOr(&holds[c], f);
+            if (near) atomicOr(&big[c * kBits + r / 32], 1u << (r % 32));
+        }
     }
     __syncthreads();
     bool apart = false;
@@ -307,8 +323,22 @@ __device__ __forceinline__ bool fx_spec_tile(const PassDesc& d, uint32_t tile, u
 #pragma unroll
     for (int g = 0; g < G; ++g) {
         // (a chirp turns every element, so nothing stays apart)
-        rare = rare || fx_tiny(words[c[g]]) ||
-               (!chirp && words[c[g]] != 0 && both[c[g]] < fx_near(words[c[g]], fx_span(R, P)));
+        {
+            const uint32_t most = words[c[g]], near = fx_near(most, fx_span(R, P));
+            bool look = !chirp && most != 0 && both[c[g]] < near;
+            if (!lane_mode && __any_sync(0xffffffffu, look)) {
+                // real values, the usual lanes without such an element: neighbouring
+                // threads hold neighbouring elements
+                uint32_t big = 0, im = 0;
+#pragma unroll
+                for (int q = 0; q < P; ++q) {
+                    big |= uint32_t(fx_mag(raw[g][q].x) >= near) << q;
+                    im |= fx_mag(raw[g][q].y) | uint32_t(__double2loint(raw[g][q].y));
+                }
+                if ((big & __shfl_xor_sync(0xffffffffu, big, 1)) && !im) look = false;
+            }
+            rare = rare || look || fx_tiny(most);
+        }
         {
             const int field = int(words[c[g]] >> 20);
             const int emax = field ? field : 4096;  // a lane of zeros: everything shifts out

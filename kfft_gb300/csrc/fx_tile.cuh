@@ -29,9 +29,10 @@
 // whose largest is below 2^-767 is left to the FP64 body, which treats them as
 // IEEE arithmetic does (smaller values beside larger ones shift out), and so is
 // one with a lane whose small parts doubles would keep apart from its large
-// ones (fx_apart in fx_math.cuh).  Telling the lanes costs 1 to 2% (4096 x 256
-// both ways 51.4 -> 51.7 us, uneven batch of 256 826 -> 841); real values in
-// the complex form take the closer look (4096 x 1024 points 70.6 -> 91.6).
+// ones (fx_apart in fx_math.cuh).  Telling the lanes costs up to 6% (4096 x 1024
+// points 69.0 -> 74.1 us, 4096 x 1000 115 -> 119, uneven batch of 256 826 ->
+// 841); real values in the complex form take 75 and, where the closer look
+// goes over them, 136.
 #pragma once
 
 #include "fft_device.cuh"
@@ -186,13 +187,22 @@ __device__ __forceinline__ bool fx_read(const PassDesc& d, cfx_t* buf, uint32_t*
         // the raw doubles to shared memory, the largest of each lane to words,
         // the largest of the smaller parts to both
         FxWalk w(d, lane_mode);
-        uint32_t seen = w.c, most = 0, most2 = 0;
-        auto flush = [&] {
-            if (most) atomicMax(&words[seen], most);
-            if (most2) atomicMax(&both[seen], most2);
+        uint32_t most = 0, most2 = 0;  // one lane: kept to the end
+        auto note = [&](uint32_t c, uint32_t m, uint32_t m2) {
+            // a warp whose elements are all of one lane sends one maximum (32
+            // atomics to one word take turns)
+            if (!lane_mode && __all_sync(0xffffffffu, c == __shfl_sync(0xffffffffu, c, 0))) {
+                m = __reduce_max_sync(0xffffffffu, m);
+                m2 = __reduce_max_sync(0xffffffffu, m2);
+                if (threadIdx.x & 31) return;
+            }
+            if (m) atomicMax(&words[c], m);
+            if (m2) atomicMax(&both[c], m2);
         };
+        // (every thread makes as many rounds: the warps vote in them)
 #pragma unroll 1
-        for (uint32_t i = threadIdx.x; i < elems; i += U * blockDim.x) {
+        for (uint32_t base = 0; base < elems; base += U * blockDim.x) {
+            const uint32_t i = base + threadIdx.x;
             double2 v[U];
             uint32_t c[U], at[U];
 #pragma unroll
@@ -214,26 +224,21 @@ __device__ __forceinline__ bool fx_read(const PassDesc& d, cfx_t* buf, uint32_t*
             }
 #pragma unroll
             for (int u = 0; u < U; ++u) {
-                if (i + u * blockDim.x >= elems) break;
-                reinterpret_cast<double2*>(buf)[at[u]] = v[u];
+                if (base + u * blockDim.x >= elems) break;
+                if (i + u * blockDim.x < elems) reinterpret_cast<double2*>(buf)[at[u]] = v[u];
                 const uint32_t a = fx_mag(v[u].x), b = fx_mag(v[u].y);
                 uint32_t m = max(a, b);
                 if (m == 0 && (__double2loint(v[u].x) | __double2loint(v[u].y))) m = 1;
                 any = max(any, m);
-                if (c[u] != seen) {
-                    flush();
-                    seen = c[u];
-                    most = most2 = 0;
+                if (d.C == 1) {
+                    most = max(most, m);
+                    most2 = max(most2, min(a, b));
+                } else {
+                    note(c[u], m, min(a, b));
                 }
-                most = max(most, m);
-                most2 = max(most2, min(a, b));
             }
         }
-        if (d.C == 1) {
-            most = __reduce_max_sync(0xffffffffu, most);
-            most2 = __reduce_max_sync(0xffffffffu, most2);
-        }
-        if (d.C > 1 || (threadIdx.x & 31) == 0) flush();
+        if (d.C == 1) note(0, most, most2);
     }
     if (__syncthreads_or((any >> 20) >= kFxExpHigh)) return false;
     // (a chirp turns every element, so nothing stays apart)
