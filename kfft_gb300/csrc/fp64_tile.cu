@@ -1,15 +1,112 @@
-// fp64_tile.cu -- the double build's IEEE arithmetic register tile, for the
+// fp64_tile.cu -- the double build's IEEE arithmetic register tiles, for the
 // tiles its fixed-point kernels turn down (an infinity, a NaN, magnitudes
-// near the ends of the exponent range).  One copy, linked to every kernel
-// that needs it, compiled for 64 registers (it may spill: it hardly ever
-// runs).
+// near the ends of the exponent range, small parts that doubles keep apart
+// from large ones).  One copy, linked to every kernel that needs it, compiled
+// for 64 registers.
 #include "fft_device.cuh"
-#include "fx_tile.cuh"
+#include "fx_spec.cuh"
 
 namespace kfft {
 #if !defined(KFFT_HALF_SCALAR)
+
+// The stages of fx_spec_tile in doubles: radix 8 with 8 points a thread, which
+// fits the 64 registers of its kernels.  The run-time body with its stages of
+// up to 16 spilled there and took, forward, with every tile in FP64, 145 us for
+// 256 x 4096 points (105 before the fixed-point tiles), 380 (275) for 4096 x
+// 1024 and 809 (577) for 16 x 2^18.
+template <uint32_t R, uint32_t NS, bool INV>
+__device__ __forceinline__ void fp64_spec_later(const PassDesc& d, double2* buf, uint32_t lane0,
+                                                uint32_t total) {
+    constexpr int P = fx_spec_radix(R, NS);
+    constexpr int G = 8 / P;
+    constexpr uint32_t M = R / P, TWS = R / (NS * P);
+    constexpr bool kLast = NS * P == R;
+    const uint32_t items = d.C * M;
+    const bool lane_mode = kLast && d.store_mode == MODE_LANE;
+    uint32_t c[G], jj[G];
+    double2 v[G][P];
+    __syncthreads();
+#pragma unroll
+    for (int g = 0; g < G; ++g) {
+        // threads past the last butterfly repeat it without storing
+        const uint32_t it = min(threadIdx.x + g * blockDim.x, items - 1);
+        jj[g] = lane_mode ? fdiv(it, d.div_C) : it % M;
+        c[g] = lane_mode ? it - jj[g] * d.C : it / M;
+        const double2* s = buf + c[g] * d.lane_stride;
+#pragma unroll
+        for (int q = 0; q < P; ++q) v[g][q] = s[pad(jj[g] + q * M)];
+        apply_inner_twiddles<P>(v[g], d.tw_inner, (jj[g] % NS) * TWS);
+        dft<P, INV>(v[g]);
+    }
+    if constexpr (!kLast) __syncthreads();
+#pragma unroll
+    for (int g = 0; g < G; ++g) {
+        if (threadIdx.x + g * blockDim.x >= items) continue;
+        const uint32_t ob = jj[g] % NS + (jj[g] / NS) * (NS * P);
+        if constexpr (kLast) {
+            if (lane0 + c[g] >= total) continue;
+            uint32_t b, j;
+            fx_lane(d, lane0 + c[g], b, j);
+            fused_store<P>(d, b, j, ob, NS, v[g]);
+        } else {
+            double2* o = buf + c[g] * d.lane_stride;
+#pragma unroll
+            for (int q = 0; q < P; ++q) o[pad(ob + q * NS)] = v[g][q];
+        }
+    }
+    if constexpr (!kLast) fp64_spec_later<R, NS * P, INV>(d, buf, lane0, total);
+}
+
+template <uint32_t R, bool INV>
+__device__ __noinline__ void fp64_spec_tile(const PassDesc& d, uint32_t tile, unsigned char* smem) {
+    constexpr int P = fx_spec_radix(R, 1);
+    constexpr int G = 8 / P;
+    constexpr uint32_t M = R / P;
+    const uint32_t total = d.batch * d.lanes_j, lane0 = tile * d.C, items = d.C * M;
+    double2* buf = reinterpret_cast<double2*>(smem);
+    const bool lane_mode = d.load_mode == MODE_LANE;
+#pragma unroll
+    for (int g = 0; g < G; ++g) {
+        const uint32_t it = threadIdx.x + g * blockDim.x;
+        if (it >= items) continue;
+        const uint32_t jj = lane_mode ? fdiv(it, d.div_C) : it % M;
+        const uint32_t c = lane_mode ? it - jj * d.C : it / M;
+        double2 v[P];
+#pragma unroll
+        for (int q = 0; q < P; ++q) v[q] = {0.0, 0.0};
+        if (lane0 + c < total) {
+            uint32_t b, j;
+            fx_lane(d, lane0 + c, b, j);
+            fused_load<P>(d, b, j, jj, M, v);
+        }
+        dft<P, INV>(v);
+        double2* o = buf + c * d.lane_stride;
+#pragma unroll
+        for (int q = 0; q < P; ++q) o[pad(jj * P + q)] = v[q];
+    }
+    fp64_spec_later<R, P, INV>(d, buf, lane0, total);
+}
+
+template <uint32_t R>
+__device__ __forceinline__ void fp64_spec(const PassDesc& d, uint32_t tile, unsigned char* smem) {
+    if (d.inv) fp64_spec_tile<R, true>(d, tile, smem);
+    else fp64_spec_tile<R, false>(d, tile, smem);
+}
+
 __device__ __noinline__ void fp64_tile(const PassDesc& d, const PassExtra& x, uint32_t tile,
                                        unsigned char* smem) {
+    switch (d.spec) {
+        case 4: fp64_spec<16>(d, tile, smem); return;
+        case 5: fp64_spec<32>(d, tile, smem); return;
+        case 6: fp64_spec<64>(d, tile, smem); return;
+        case 7: fp64_spec<128>(d, tile, smem); return;
+        case 8: fp64_spec<256>(d, tile, smem); return;
+        case 9: fp64_spec<512>(d, tile, smem); return;
+        case 10: fp64_spec<1024>(d, tile, smem); return;
+        case 11: fp64_spec<2048>(d, tile, smem); return;
+        case 12: fp64_spec<4096>(d, tile, smem); return;
+        default: break;
+    }
     vec2_t* sm = reinterpret_cast<vec2_t*>(smem);
     if (d.inv) tile_body_reg<true, false, false>(d, x, tile, sm);
     else tile_body_reg<false, false, false>(d, x, tile, sm);
