@@ -284,7 +284,11 @@ void launch_pass_reg(const PassDesc& d, const PassExtra& x, cudaStream_t st) {
             const int per_sm = f ? prepare((const void*)f, smem) : -1;
             const uint32_t grid = uint32_t(std::max(per_sm, 0)) * uint32_t(sm_count());
             uint32_t* fail = wait_flags();
-            if (fail && per_sm > 0 && d.tiles >= 2 * grid) {
+            // from where k_pass_pipe's two CTAs an SM start a third round (608
+            // tiles; us there and here: 16 points 700 tiles 20.6, 18.0, 760 tiles
+            // 24.7, 20.6, 911 tiles 24.7, 20.6; 256 points 760 tiles 12.4, 10.4;
+            // 4096 points level; at 608 tiles 12.4, 14.4)
+            if (fail && per_sm > 0 && 3 * d.tiles > 4 * grid) {
                 f<<<grid, kPassThreads, smem, st>>>(d, fail + wait_slot(), bulk_wait_polls());
                 note_cuda_error(cudaGetLastError());
                 note_bulk_launch();
@@ -305,7 +309,9 @@ void launch_pass_reg(const PassDesc& d, const PassExtra& x, cudaStream_t st) {
                 (d.C * d.R + d.C * d.lane_stride + 1u) * uint32_t(sizeof(vec2_t));
             const int per_sm = f ? prepare((const void*)f, smem) : -1;
             const uint32_t grid = uint32_t(std::max(per_sm, 0)) * uint32_t(sm_count());
-            if (per_sm > 0 && d.tiles >= 2 * grid) {
+            // from 760 tiles on (us of k_pass_pipe and here: 2^20 points 768 tiles 44.8,
+            // 39.1, 2^18 31.8, 30.9, 2^13 26.8, 23.1; at 704 tiles 2^18 28.8, 30.9)
+            if (per_sm > 0 && 3 * d.tiles >= 5 * grid) {
                 f<<<grid, kPassThreads, smem, st>>>(d, pairs ? 1u : 0u);
                 note_cuda_error(cudaGetLastError());
                 count_launch();
