@@ -135,7 +135,7 @@ struct PassDesc {
 #if !defined(KFFT_HALF_SCALAR)
     // fixed-point tile (fx_tile.cuh): forward tables in two-limb form
     uint8_t fx;             // the tile runs in fixed point
-    uint8_t inplace;        // three or more stages of one butterfly a thread: one exchange buffer
+    uint8_t inplace;        // every stage one round of butterflies: one exchange buffer
     uint32_t fx_words;      // byte offsets of the lane words and the lane table in shared memory
     uint32_t fx_lanes;
     const FxTw* fx_inner;   // tw_inner's forward twiddles

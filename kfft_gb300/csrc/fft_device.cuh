@@ -634,8 +634,9 @@ __device__ __forceinline__ void tile_body(const PassDesc& d, const PassExtra& x,
 // ---------------------------------------------------------------------------
 enum : int { IO_SMEM = 0, IO_GLOBAL = 1 };
 
-// v[q] *= W^(q*step) for q = 1..P-1, W^i = tw[i].  FP64 loads every factor
-// (the FP64 pipe, not the loads, bounds it).  FP32 loads the four anchors
+// v[q] *= W^(q*step) for q = 1..P-1, W^i = tw[i].  In doubles (the FP64 tiles
+// behind the fixed-point ones) every factor is loaded: the FP64 pipe, not the
+// loads, bounds them.  FP32 loads the four anchors
 // W^(step), W^(2 step), W^(4 step), W^(8 step) and forms the others as
 // products of at most four anchors: a quarter of the table loads, which were
 // the L1 bottleneck, for a few ulp of extra rounding.
@@ -862,10 +863,6 @@ __device__ __forceinline__ void fused_store(const PassDesc& d, uint32_t bs, uint
     }
 }
 
-// One inner Stockham pass of radix P over the tile: each thread takes one
-// butterfly at a time from `src` (global memory on the first pass, else a
-// shared buffer) and writes it to `dst` (global memory on the last pass, else
-// the other shared buffer).
 // LIN: element i of a lane lies at slot i of its shared-memory lane (run-time
 // FP32 tiles: an address is a base plus q steps), else at pad(i).
 template <bool LIN>
@@ -905,6 +902,10 @@ __device__ __forceinline__ void exchange_pass(const PassDesc& d, const InnerStep
 }
 #endif
 
+// One inner Stockham pass of radix P over the tile: each thread takes one
+// butterfly at a time from `src` (global memory on the first pass, else a
+// shared buffer) and writes it to `dst` (global memory on the last pass, else
+// the other shared buffer).
 template <int P, bool INV, int STORE, bool LIN>
 __device__ __forceinline__ void fused_pass(const PassDesc& d, const InnerStep& st,
                                            const vec2_t* src, vec2_t* dst, uint32_t lane0,

@@ -6,9 +6,20 @@
 // 0.60 T/s DFMA, 18.9 T/s mad.wide, 19.0 T/s add.s64), so the double build
 // computes its butterflies in 64-bit integers: the values of one lane (one
 // sub-FFT of a tile) share a power-of-two scale that follows the lane's
-// largest value from stage to stage, with 60 or so significant bits for that
-// value against the 53 of a double.  Additions are exact; every product keeps
-// 2^-62 of the lane's scale.  Inputs and outputs stay doubles.
+// largest value from stage to stage.  Inputs and outputs stay doubles.
+//
+// What is kept, in units of the lane's scale: an input's leading bit lies at 59
+// for the lane's largest part (58 before a first stage of radix 5 to 8, 57
+// before one of 9 to 16), and what falls below one unit is cut off; behind a
+// chirp or an outer twiddle it lies at 61 (60, 59) and the product, a quarter of
+// the true one, is whole units.  Later stages shift the lane's largest part up
+// to 60 or 61 (less the radix's room) before their twiddles, whose products
+// again are quarters in whole units.  Additions are exact.  So the largest part
+// has 57 to 60 significant bits against the 53 of a double, and a smaller one
+// as many fewer as it is smaller: the error is a few units whatever a value's
+// size, below a double's in the norm of the lane but not for a part that
+// nothing large is added to.  Lanes with such parts are found and left to
+// arithmetic in doubles (fx_apart below).
 //
 // A real number x in [-1, 1] that multiplies data (a twiddle's part) is held
 // as x * 2^62 in two signed 32-bit limbs, hi * 2^32 + lo with lo in

@@ -29,9 +29,11 @@ BulkKernel bulk_kernel(uint32_t spec, bool inv, bool plain);
 
 // FP32 power-of-two passes, one kernel per pass length R so each kernel holds
 // only its own body (a small instruction footprint):
-// * k_pass_async: a plain prologue, full tiles of lanes in rows and more tiles
+// * k_pass_bulk: whole contiguous sequences, a plain prologue and more tiles
 //   than fit the GPU at once: a grid of resident CTAs, each running many tiles
-//   with its next tile on its way into shared memory (tile_loop_async);
+//   with its next one on its way by a bulk copy (tile_loop_bulk);
+// * k_pass_async: the same for full tiles of lanes in rows, the next tile on its
+//   way by asynchronous copies (tile_loop_async);
 // * k_pass_pipe: the same for other tiles, the next tile's loads in registers
 //   (tile_loop_pipelined);
 // * k_pass_spec: one tile per CTA otherwise.
@@ -150,7 +152,8 @@ template <bool INV, int STORE, bool TC, int BLOCKS>
 __global__ void __launch_bounds__(kPassThreads, BLOCKS) k_pass_reg(const __grid_constant__ PassDesc d,
                                                               const __grid_constant__ PassExtra x) {
     extern __shared__ __align__(16) unsigned char smem_raw[];
-    // power-of-two FP32 passes launch k_pass_spec / k_pass_pipe instead
+    // power-of-two passes launch k_pass_bulk, k_pass_async, k_pass_pipe or
+    // k_pass_spec instead
     tile_body_reg<INV, false, TC, STORE>(d, x, blockIdx.x, reinterpret_cast<vec2_t*>(smem_raw));
 }
 

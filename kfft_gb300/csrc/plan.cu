@@ -144,7 +144,11 @@ constexpr uint32_t kRegLanes = 4;
 // true when a tile of C lanes of length R fits the fused-I/O kernel: every
 // inner radix <= 16 and at most kRegTile points per tile
 // (double build: and, where the plan limits the threads of a tile, at most one
-// round of butterflies in every stage, so that one exchange buffer does)
+// round of butterflies in every stage, so that one exchange buffer does.  In the
+// queue, with 256 threads, a radix-7 stage over more than 1792 points does not
+// fit, nor one of 448 points in four lanes: those lengths take a pass more.  512
+// sequences of 1792 points 84 us, in one FP64 pass 136; 1960 77 and 178, 2016 68
+// and 168; 8 of 512 x 448 160 and 378)
 static bool reg_tile_fits(uint32_t R, uint32_t C, uint32_t cap = kRegTile,
                           uint32_t fx_threads = kFxWideThreads) {
     if (C < 1 || uint64_t(C) * R > std::min(cap, kRegTile)) return false;
@@ -654,11 +658,9 @@ static PassDesc make_desc(const FftPlan& P, size_t pi, const vec2_t* in, const L
     while (!d.regmode && C > 1 && smem_for(C * s.R) > kSmemBudget) --C;
     d.C = C;
     // power-of-two register tiles of 16..4096 points run a compile-time body
-    // (FP32 only: in FP64 its fully unrolled stages spill and the FP64 pipe,
-    // not index arithmetic, bounds the pass)
     d.spec = 0;
 #if !defined(KFFT_HALF_SCALAR)
-    // power-of-two passes run fx_spec_tile: 8 points a thread
+    // (fx_spec_tile: 8 points a thread)
     if (d.regmode && s.R >= 16 && s.R <= 4096 && (s.R & (s.R - 1)) == 0 &&
         C * s.R <= 8 * P.var.fx_threads) {
         uint32_t l = 0;
