@@ -112,11 +112,8 @@ constexpr __host__ __device__ int fx_room(int P) { return P <= 4 ? 0 : (P <= 8 ?
 
 // How many bits below the largest a part may lie and still count as near it:
 // up to 7 it is held to its last bit (the leading bit at 59, 53 bits), less the
-// room of the first radix; two bits stricter where the cut-off bits of many
-// elements add up.
-__host__ __device__ constexpr int fx_span(uint32_t R, int P) {
-    return (R < 64 ? 7 : 5) - fx_room(P);
-}
+// room of the first radix.
+__host__ __device__ constexpr int fx_span(int P) { return 7 - fx_room(P); }
 // magnitude words (the high word of a double without its sign) from this one
 // on are near the largest, `most`
 __host__ __device__ constexpr uint32_t fx_near(uint32_t most, int span) {

@@ -205,7 +205,7 @@ __device__ __forceinline__ bool fx_spec_apart(const PassDesc& d, uint32_t* words
             uint32_t n = j + r * d.lanes_j;
             if (d.pro_op == PRO_GATHER) n = __ldg(&d.pro_perm[n]);
             const double2 x = __ldcg(&d.in[uint64_t(b) * d.in_bs + uint64_t(n) * d.in_es]);
-            const uint32_t from = fx_near(words[c], fx_span(R, fx_spec_radix(R, 1)));
+            const uint32_t from = fx_near(words[c], fx_span(fx_spec_radix(R, 1)));
             f = fx_holds(x, from);
             near = max(fx_mag(x.x), fx_mag(x.y)) >= from;
         }
@@ -324,7 +324,7 @@ __device__ __forceinline__ bool fx_spec_tile(const PassDesc& d, uint32_t tile, u
     for (int g = 0; g < G; ++g) {
         // (a chirp turns every element, so nothing stays apart)
         {
-            const uint32_t most = words[c[g]], near = fx_near(most, fx_span(R, P));
+            const uint32_t most = words[c[g]], near = fx_near(most, fx_span(P));
             bool look = !chirp && most != 0 && both[c[g]] < near;
             if (!lane_mode && __any_sync(0xffffffffu, look)) {
                 // real values, the usual lanes without such an element: neighbouring

@@ -242,7 +242,7 @@ __device__ __forceinline__ bool fx_read(const PassDesc& d, cfx_t* buf, uint32_t*
     if (__syncthreads_or((any >> 20) >= kFxExpHigh)) return false;
     // (a chirp turns every element, so nothing stays apart)
     const bool chirped = d.pro_op == PRO_CHIRP;
-    const int span = fx_span(d.R, d.rad[0]);
+    const int span = fx_span(d.rad[0]);
     bool rare = false, tiny = false;
     for (uint32_t c = threadIdx.x; c < d.C; c += blockDim.x) {
         tiny = tiny || fx_tiny(words[c]);

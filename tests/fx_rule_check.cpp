@@ -44,7 +44,7 @@ int main() {
         uint32_t most = 0, holds = 0;
         for (int i = 0; i < n; ++i) most = std::max(most, std::max(mag(re[i]), mag(im[i])));
         if (!most) continue;
-        const int span = fx_span(uint32_t(n), n % 16 == 0 ? 4 : 16);
+        const int span = fx_span(n % 16 == 0 ? 4 : 16);
         const uint32_t near = fx_near(most, span);
         for (int i = 0; i < n; ++i) {
             const int k = (i + 1) % n;
@@ -76,10 +76,7 @@ int main() {
     }
     // a part within the span of the largest keeps all its 53 bits
     for (int P = 2; P <= 16; ++P)
-        for (uint32_t R : {8u, 63u, 64u, 4096u}) {
-            const int top = 59 - fx_room(P);
-            if (top - fx_span(R, P) < 52) ++exact_lost;
-        }
+        if (59 - fx_room(P) - fx_span(P) < 52) ++exact_lost;
     std::printf("%ld %ld %ld %ld\n", stay, leave, wrong, exact_lost);
     return 0;
 }
