@@ -9,6 +9,79 @@
 namespace kfft {
 #if !defined(KFFT_HALF_SCALAR)
 
+// The lanes' elements are read again.  Behind the rows of words one for what
+// each lane holds and a bit an element that is near its lane's largest.
+__device__ __noinline__ bool fx_spec_apart(const PassDesc& d, uint32_t R, uint32_t* words, uint32_t lane0,
+                                           uint32_t total, int span) {
+    bool beyond = false;
+    for (uint32_t c = threadIdx.x; c < d.C; c += blockDim.x) beyond = beyond || fx_beyond(words[c]);
+    if (__syncthreads_or(beyond)) return true;
+    constexpr int U = 4;  // loads in flight together
+    const uint32_t log = d.spec, bits = (R + 31) / 32;
+    uint32_t* holds = words + (kFxRows + 1) * d.C;
+    uint32_t* big = holds + d.C;
+    const bool lane_mode = d.load_mode == MODE_LANE;
+    // rows of 32 elements or more, element by element: a warp has one lane's and
+    // a word of bits (whole warps: C * R and the threads are multiples of 32)
+    const bool by_warp = R >= 32 && !lane_mode;
+    const uint32_t elems = d.C * R;
+#pragma unroll 1
+    for (uint32_t i0 = threadIdx.x; i0 < elems; i0 += U * blockDim.x) {
+        double2 x[U];
+        uint32_t at[U];  // the element's bit, lane by lane (none: past the last)
+#pragma unroll
+        for (int u = 0; u < U; ++u) {
+            const uint32_t i = i0 + u * blockDim.x;
+            const uint32_t r = lane_mode ? fdiv(i, d.div_C) : i & (R - 1);
+            const uint32_t c = lane_mode ? i - r * d.C : i >> log;
+            x[u] = {0.0, 0.0};
+            at[u] = 0xffffffffu;
+            if (i < elems) {
+                at[u] = (c << log) + r;
+                if (lane0 + c < total) {
+                    uint32_t b, j;
+                    fx_lane(d, lane0 + c, b, j);
+                    uint32_t n = j + r * d.lanes_j;
+                    if (d.pro_op == PRO_GATHER) n = __ldg(&d.pro_perm[n]);
+                    x[u] = __ldcg(&d.in[uint64_t(b) * d.in_bs + uint64_t(n) * d.in_es]);
+                }
+            }
+        }
+#pragma unroll
+        for (int u = 0; u < U; ++u) {
+            if (at[u] == 0xffffffffu) break;  // (whole warps)
+            const uint32_t c = at[u] >> log, r = at[u] & (R - 1);
+            const uint32_t from = fx_near(words[c], span);
+            uint32_t f = fx_holds(x[u], from);
+            const bool near = max(fx_mag(x[u].x), fx_mag(x[u].y)) >= from;
+            if (by_warp) {
+                f = __reduce_or_sync(0xffffffffu, f);
+                const uint32_t w = __ballot_sync(0xffffffffu, near);
+                if ((threadIdx.x & 31) == 0) {
+                    if (f) atomicOr(&holds[c], f);
+                    big[c * bits + r / 32] = w;
+                }
+            } else {
+                if (f) atomicOr(&holds[c], f);
+                if (near) atomicOr(&big[c * bits + r / 32], 1u << (r % 32));
+            }
+        }
+    }
+    __syncthreads();
+    bool apart = false;
+    for (uint32_t c = threadIdx.x; c < d.C; c += blockDim.x) {
+        uint32_t f = holds[c];
+        const uint32_t* w = big + c * bits;
+        for (uint32_t k = 0; k < bits && fx_apart(f); ++k) {
+            // bit r with bit r + 1 (the first one behind the last)
+            const uint32_t up = w[k + 1 < bits ? k + 1 : 0] & 1u;
+            if (w[k] & ((w[k] >> 1) | up << (R < 32 ? R - 1 : 31))) f |= FX_PAIR;
+        }
+        apart = apart || fx_apart(f);
+    }
+    return __syncthreads_or(apart);
+}
+
 // The stages of fx_spec_tile in doubles: radix 8 with 8 points a thread, which
 // fits the 64 registers of its kernels.  The run-time body with its stages of
 // up to 16 spilled there and took, forward, with every tile in FP64, 145 us for

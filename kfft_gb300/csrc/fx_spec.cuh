@@ -177,64 +177,12 @@ __device__ __forceinline__ void fx_spec_later(const PassDesc& d, cfx_t* buf, uin
     }
 }
 
-// The closer look at a tile with a lane that may need the FP64 body (fx_tiny,
-// fx_apart): its elements read again.  Behind the rows of words one for what each lane
-// holds and a bit an element that is near its lane's largest.
-template <uint32_t R>
-__device__ __forceinline__ bool fx_spec_apart(const PassDesc& d, uint32_t* words, uint32_t lane0,
-                                              uint32_t total) {
-    constexpr uint32_t kBits = (R + 31) / 32;
-    uint32_t* holds = words + (kFxRows + 1) * d.C;
-    uint32_t* big = holds + d.C;
-    const bool lane_mode = d.load_mode == MODE_LANE;
-    bool tiny = false;
-    for (uint32_t c = threadIdx.x; c < d.C; c += blockDim.x) tiny = tiny || fx_tiny(words[c]);
-    if (__syncthreads_or(tiny)) return true;
-    // rows of 32 elements or more, element by element: a warp has one lane's and
-    // a word of bits (whole warps: C * R and the threads are multiples of 32)
-    const bool by_warp = R >= 32 && !lane_mode;
-#pragma unroll 4
-    for (uint32_t i = threadIdx.x; i < d.C * R; i += blockDim.x) {
-        const uint32_t r = lane_mode ? fdiv(i, d.div_C) : i % R;
-        const uint32_t c = lane_mode ? i - r * d.C : i / R;
-        uint32_t f = 0;
-        bool near = false;
-        if (lane0 + c < total && words[c] != 0) {
-            uint32_t b, j;
-            fx_lane(d, lane0 + c, b, j);
-            uint32_t n = j + r * d.lanes_j;
-            if (d.pro_op == PRO_GATHER) n = __ldg(&d.pro_perm[n]);
-            const double2 x = __ldcg(&d.in[uint64_t(b) * d.in_bs + uint64_t(n) * d.in_es]);
-            const uint32_t from = fx_near(words[c], fx_span(fx_spec_radix(R, 1)));
-            f = fx_holds(x, from);
-            near = max(fx_mag(x.x), fx_mag(x.y)) >= from;
-        }
-        if (by_warp) {
-            f = __reduce_or_sync(0xffffffffu, f);
-            const uint32_t bits = __ballot_sync(0xffffffffu, near);
-            if ((threadIdx.x & 31) == 0) {
-                if (f) atomicOr(&holds[c], f);
-                big[c * kBits + r / 32] = bits;
-            }
-        } else {
-            if (f) atomicOr(&holds[c], f);
-            if (near) atomicOr(&big[c * kBits + r / 32], 1u << (r % 32));
-        }
-    }
-    __syncthreads();
-    bool apart = false;
-    for (uint32_t c = threadIdx.x; c < d.C; c += blockDim.x) {
-        uint32_t f = holds[c];
-        const uint32_t* w = big + c * kBits;
-        for (uint32_t k = 0; k < kBits && fx_apart(f); ++k) {
-            // bit r with bit r + 1 (the first one behind the last)
-            const uint32_t up = w[k + 1 < kBits ? k + 1 : 0] & 1u;
-            if (w[k] & ((w[k] >> 1) | up << (R < 32 ? R - 1 : 31))) f |= FX_PAIR;
-        }
-        apart = apart || fx_apart(f);
-    }
-    return __syncthreads_or(apart);
-}
+// The closer look at a tile of lanes of R points (a power of two) with one that
+// may need the FP64 body (fx_beyond, fx_apart): true if one does.  In fp64_tile.cu,
+// out of the way of the other tiles' code (65536 x 64 points 48.1 us with it in
+// line, 46.4 so; 320 x 8192 96.8 and 93.0).
+__device__ bool fx_spec_apart(const PassDesc& d, uint32_t R, uint32_t* words, uint32_t lane0, uint32_t total,
+                              int span);
 
 // One tile (C * R <= 8 points a thread); false (with nothing written) when it
 // is one for the FP64 body.
@@ -253,7 +201,6 @@ __device__ __forceinline__ bool fx_spec_tile(const PassDesc& d, uint32_t tile, u
     const bool lane_mode = d.load_mode == MODE_LANE;
     uint32_t c[G], jj[G];
     double2 raw[G][P];
-    bool bad = false;
 #pragma unroll
     for (int g = 0; g < G; ++g) {
         // threads past the last butterfly repeat it without storing
@@ -298,24 +245,26 @@ __device__ __forceinline__ bool fx_spec_tile(const PassDesc& d, uint32_t tile, u
             const int x = __double2hiint(raw[g][q].x), y = __double2hiint(raw[g][q].y);
             neg = __vimax3_u32(neg, uint32_t(x), uint32_t(y));
             pos = __vimax3_s32(pos, x, y);
-            // (two elements of each butterfly show nearly every lane that stays)
+            // (two elements of some butterflies show nearly every lane that stays)
             if (q == 0 || q == P / 2) m2 = max(m2, min(uint32_t(x) & 0x7fffffffu, uint32_t(y) & 0x7fffffffu));
             low |= uint32_t(__double2loint(raw[g][q].x)) | uint32_t(__double2loint(raw[g][q].y));
         }
         uint32_t m = max(neg & 0x7fffffffu, uint32_t(pos));
         if (m == 0 && low) m = 1;
-        bad = bad || (m >> 20) >= kFxExpHigh;
         if (M % 32 == 0 && !lane_mode) {
             m = __reduce_max_sync(0xffffffffu, m);
-            m2 = __reduce_max_sync(0xffffffffu, m2);
             if ((threadIdx.x & 31) == 0 && m) atomicMax(&words[c[g]], m);
-            if ((threadIdx.x & 31) == 0 && m2) atomicMax(&both[c[g]], m2);
+            if (jj[g] < 32) {  // (one warp of the lane)
+                m2 = __reduce_max_sync(0xffffffffu, m2);
+                if ((threadIdx.x & 31) == 0 && m2) atomicMax(&both[c[g]], m2);
+            }
         } else {
+            constexpr uint32_t kSome = M >= 16 ? 3 : (M >= 8 ? 1 : 0);  // (four butterflies or so)
             atomicMax(&words[c[g]], m);
-            atomicMax(&both[c[g]], m2);
+            if ((jj[g] & kSome) == 0) atomicMax(&both[c[g]], m2);
         }
     }
-    if (__syncthreads_or(bad)) return false;
+    __syncthreads();
     const bool outer = d.Ns > 1, chirp = d.pro_op == PRO_CHIRP, inv = d.inv != 0;
     const int top = (outer || chirp ? 61 : 59) - fx_room(P);
     bool rare = false;
@@ -337,7 +286,7 @@ __device__ __forceinline__ bool fx_spec_tile(const PassDesc& d, uint32_t tile, u
                 }
                 if ((big & __shfl_xor_sync(0xffffffffu, big, 1)) && !im) look = false;
             }
-            rare = rare || look || fx_tiny(most);
+            rare = rare || look || fx_beyond(most);
         }
         {
             const int field = int(words[c[g]] >> 20);
@@ -372,7 +321,8 @@ __device__ __forceinline__ bool fx_spec_tile(const PassDesc& d, uint32_t tile, u
         }
     }
     fx_spec_exchange<P, G, R, 1>(d, buf, words + d.C, c, jj, v, lane_mode);
-    if (__syncthreads_or(rare) && fx_spec_apart<R>(d, words, lane0, total)) return false;
+    if (__builtin_expect(__syncthreads_or(rare), 0) && fx_spec_apart(d, R, words, lane0, total, fx_span(P)))
+        return false;
     fx_spec_later<R, P, 1>(d, buf, words, lane0, total);
     return true;
 }

@@ -28,10 +28,12 @@
 // whose largest is below 2^-767 is left to the FP64 body, which treats them as
 // IEEE arithmetic does (smaller values beside larger ones shift out), and so is
 // one with a lane whose small parts doubles would keep apart from its large
-// ones (fx_apart in fx_math.cuh).  Telling the lanes costs up to 6% (4096 x 1024
-// points 69.0 -> 74.1 us, 4096 x 1000 115 -> 119, uneven batch of 256 826 ->
-// 841); real values in the complex form take 75 and, where the closer look
-// goes over them, 136.
+// ones (fx_apart in fx_math.cuh).  Telling the lanes costs up to 6% (65536 x 64
+// points 43.8 -> 46.4 us, 4096 x 1000 116 -> 119, uneven batch of 256 829 -> 842,
+// 4096^2 both ways level); real values in the complex form, 4096 x 1000 points,
+// take the closer look and 136; a tile that leaves after it has spent 10 to 15% of
+// its FP64 time (256 x 4096 nearly real points 121 us, in FP64 from the start
+// 106).
 #pragma once
 
 #include "fft_device.cuh"
@@ -43,7 +45,9 @@ namespace kfft {
 
 // a lane's largest exponent field outside this range goes to the FP64 body
 constexpr uint32_t kFxExpLow = 256, kFxExpHigh = 1791;
-__device__ __forceinline__ bool fx_tiny(uint32_t most) { return most != 0 && (most >> 20) < kFxExpLow; }
+__device__ __forceinline__ bool fx_beyond(uint32_t most) {
+    return most != 0 && ((most >> 20) < kFxExpLow || (most >> 20) >= kFxExpHigh);
+}
 
 __device__ __forceinline__ FxTw fx_tw_load(const FxTw* p) {
     const int4 v = __ldg(reinterpret_cast<const int4*>(p));
@@ -180,7 +184,6 @@ __device__ __forceinline__ bool fx_read(const PassDesc& d, cfx_t* buf, uint32_t*
     const bool lane_mode = d.load_mode == MODE_LANE;
     const uint64_t step = uint64_t(d.lanes_j) * d.in_es;
     constexpr int U = 4;  // loads in flight together
-    uint32_t any = 0;
     uint32_t* both = words + fx_guard_row(d) * d.C;
     {
         // the raw doubles to shared memory, the largest of each lane to words,
@@ -228,7 +231,6 @@ __device__ __forceinline__ bool fx_read(const PassDesc& d, cfx_t* buf, uint32_t*
                 const uint32_t a = fx_mag(v[u].x), b = fx_mag(v[u].y);
                 uint32_t m = max(a, b);
                 if (m == 0 && (__double2loint(v[u].x) | __double2loint(v[u].y))) m = 1;
-                any = max(any, m);
                 if (d.C == 1) {
                     most = max(most, m);
                     most2 = max(most2, min(a, b));
@@ -239,17 +241,17 @@ __device__ __forceinline__ bool fx_read(const PassDesc& d, cfx_t* buf, uint32_t*
         }
         if (d.C == 1) note(0, most, most2);
     }
-    if (__syncthreads_or((any >> 20) >= kFxExpHigh)) return false;
+    __syncthreads();
     // (a chirp turns every element, so nothing stays apart)
     const bool chirped = d.pro_op == PRO_CHIRP;
     const int span = fx_span(d.rad[0]);
-    bool rare = false, tiny = false;
+    bool rare = false, beyond = false;
     for (uint32_t c = threadIdx.x; c < d.C; c += blockDim.x) {
-        tiny = tiny || fx_tiny(words[c]);
+        beyond = beyond || fx_beyond(words[c]);
         rare = rare || (!chirped && words[c] != 0 && both[c] < fx_near(words[c], span));
     }
-    if (__syncthreads_or(rare || tiny)) {
-        if (__syncthreads_or(tiny)) return false;
+    if (__syncthreads_or(rare || beyond)) {
+        if (__syncthreads_or(beyond)) return false;
         uint32_t* holds = both + d.C;
         FxWalk w(d, false);
 #pragma unroll 1
