@@ -927,15 +927,13 @@ def aggregate_over_ranks(ms_total, flops_per_step, steps, world, dist=None, devi
 # DRAM bytes per launch of the dominant kernel from ncu captures
 # (dram__bytes_read.sum + dram__bytes_write.sum, averaged over the captured
 # pass launches).  The uneven batch is too large for a full-set capture:
-# every 8th sequence was captured (37.47 M points, 2.708 GB) and scaled by
+# every 8th sequence was captured (37.47 M points, 2.714 GB, in double 6.590) and scaled by
 # points, which the same length mix allows.
-# (The double queue's figure is of its FP64 tiles; its fixed-point tiles move
-# the same data but Bluestein lengths are powers of two more often.)
-NCU_DRAM_BYTES_PER_POINT = {"uneven_float": 2.708141e9 / 37465227,
-                            "uneven_double": 5.925791e9 / 37465227}
+NCU_DRAM_BYTES_PER_POINT = {"uneven_float": 2.714176e9 / 37465227,
+                            "uneven_double": 6.590382e9 / 37465227}
 NCU_DRAM_BYTES_PER_LAUNCH = {"c2c_f32_4096x4096": 213.2e6, "c2c_f32_2p18x64": 213.6e6,
                              "c2c_f32_2p20x16": 215.7e6, "c2c_f32_2p24": 213.0e6,
-                             "c2c4096": 18.7e6}
+                             "c2c4096": 16.9e6}
 
 
 def dominant_kernel_roofline(wl, ms_step, lib, peak, peak_kind, launches_per_step=None,

@@ -22,14 +22,14 @@
 // Measured (forward, us): 4096 x 4000 points 494, against 987 with the inputs
 // held in registers, radices at 128 registers and two exchange buffers;
 // 16384 x 1000 417 against 566.  The FP64 body these tiles replace ran the
-// uneven batch of 256 in 1672 us, they run it in 851.
+// uneven batch of 256 in 1672 us, they run it in 862.
 //
 // A tile that holds an infinity, a NaN, a magnitude from 2^768 on or a lane
 // whose largest is below 2^-767 is left to the FP64 body, which treats them as
 // IEEE arithmetic does (smaller values beside larger ones shift out), and so is
 // one with a lane whose small parts doubles would keep apart from its large
 // ones (fx_apart in fx_math.cuh).  Telling the lanes costs up to 6% (65536 x 64
-// points 43.8 -> 46.4 us, 4096 x 1000 116 -> 119, uneven batch of 256 829 -> 842,
+// points 43.8 -> 46.4 us, 4096 x 1000 116 -> 119, uneven batch of 256 829 -> 862,
 // 4096^2 both ways level); real values in the complex form, 4096 x 1000 points,
 // take the closer look and 136; a tile that leaves after it has spent 10 to 15% of
 // its FP64 time (256 x 4096 nearly real points 121 us, in FP64 from the start

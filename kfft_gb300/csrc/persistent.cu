@@ -11,7 +11,7 @@ namespace kfft {
 // resident CTAs per SM of the queue kernel (its tiles are capped at 2048
 // points): four for FP32 (64 registers a thread), three for the double build
 // (80 registers; 256 sequences of up to 2^18 points, as the tiles stood: 0.89
-// ms, two CTAs 0.95, four 0.97; 0.85 now)
+// ms, two CTAs 0.95, four 0.97; 0.86 now)
 #ifndef KFFT_QUEUE_MINBLOCKS
 #if defined(KFFT_HALF_SCALAR)
 #define KFFT_QUEUE_MINBLOCKS 4
