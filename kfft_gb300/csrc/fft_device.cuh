@@ -873,17 +873,21 @@ __device__ __forceinline__ uint32_t slot(uint32_t i) {
 #if !defined(KFFT_HALF_SCALAR)
 // A middle stage in one buffer (PassDesc::inplace): at most fx_group(P)
 // butterflies a thread, all read before any is written.  Threads past the
-// last butterfly repeat it without storing.
+// last butterfly repeat it without storing.  `only`: as in fused_pass.
 template <int P, bool INV>
-__device__ __forceinline__ void exchange_pass(const PassDesc& d, const InnerStep& st, vec2_t* buf) {
+__device__ __forceinline__ void exchange_pass(const PassDesc& d, const InnerStep& st, vec2_t* buf,
+                                              const uint32_t* only) {
     constexpr int G = int(fx_group(P));
     const uint32_t m = st.m, items = d.C * m;
     vec2_t v[G][P];
     uint32_t lane[G], ob[G];
+    bool on[G];
 #pragma unroll
     for (int g = 0; g < G; ++g) {
         const uint32_t it = min(threadIdx.x + g * blockDim.x, items - 1);
         const uint32_t c = fdiv(it, st.div_m), jj = it - c * m;
+        on[g] = !only || only[c];
+        if (!on[g]) continue;
         const uint32_t blk = fdiv(jj, st.div_ns), kk = jj - blk * st.ns;
         lane[g] = c * d.lane_stride;
         ob[g] = blk * st.ns * P + kk;
@@ -895,7 +899,7 @@ __device__ __forceinline__ void exchange_pass(const PassDesc& d, const InnerStep
     __syncthreads();
 #pragma unroll
     for (int g = 0; g < G; ++g)
-        if (threadIdx.x + g * blockDim.x < items) {
+        if (on[g] && threadIdx.x + g * blockDim.x < items) {
 #pragma unroll
             for (int q = 0; q < P; ++q) buf[lane[g] + pad(ob[g] + q * st.ns)] = v[g][q];
         }
@@ -905,18 +909,21 @@ __device__ __forceinline__ void exchange_pass(const PassDesc& d, const InnerStep
 // One inner Stockham pass of radix P over the tile: each thread takes one
 // butterfly at a time from `src` (global memory on the first pass, else a
 // shared buffer) and writes it to `dst` (global memory on the last pass, else
-// the other shared buffer).
+// the other shared buffer).  `only` (if given; FP64 tiles): the lanes to do, the
+// others are left alone; consecutive threads then take one lane's butterflies,
+// as few warps as there are lanes.
 template <int P, bool INV, int STORE, bool LIN>
 __device__ __forceinline__ void fused_pass(const PassDesc& d, const InnerStep& st,
                                            const vec2_t* src, vec2_t* dst, uint32_t lane0,
-                                           uint32_t total, int sio, int dio) {
+                                           uint32_t total, int sio, int dio,
+                                           const uint32_t* only = nullptr) {
     const uint32_t m = st.m, ns = st.ns;
     const uint32_t items = d.C * m;
-    const bool cfast = (sio == IO_GLOBAL) ? (d.load_mode == MODE_LANE)
-                                          : ((dio == IO_GLOBAL) ? (d.store_mode == MODE_LANE) : false);
+    const bool cfast = !only && ((sio == IO_GLOBAL) ? (d.load_mode == MODE_LANE)
+                                                    : ((dio == IO_GLOBAL) ? (d.store_mode == MODE_LANE) : false));
 #if !defined(KFFT_HALF_SCALAR)
     if (d.inplace && sio == IO_SMEM && dio == IO_SMEM) {
-        exchange_pass<P, INV>(d, st, dst);
+        exchange_pass<P, INV>(d, st, dst, only);
         return;
     }
 #endif
@@ -929,6 +936,7 @@ __device__ __forceinline__ void fused_pass(const PassDesc& d, const InnerStep& s
             c = fdiv(it, st.div_m);
             jj = it - c * m;
         }
+        if (only && !only[c]) continue;
         const uint32_t g = lane0 + c;
         uint32_t bs = 0, j = 0;
         const bool live = g < total;
@@ -1649,23 +1657,24 @@ __device__ __forceinline__ void tile_loop_bulk(const PassDesc& d, unsigned char*
 template <bool INV, int STORE, bool LIN>
 __device__ __forceinline__ void fused_dispatch(int P, const PassDesc& d, const InnerStep& st,
                                                const vec2_t* src, vec2_t* dst, uint32_t lane0,
-                                               uint32_t total, int sio, int dio) {
+                                               uint32_t total, int sio, int dio,
+                                               const uint32_t* only) {
     switch (P) {
-        case 2: fused_pass<2, INV, STORE, LIN>(d, st, src, dst, lane0, total, sio, dio); break;
-        case 3: fused_pass<3, INV, STORE, LIN>(d, st, src, dst, lane0, total, sio, dio); break;
-        case 4: fused_pass<4, INV, STORE, LIN>(d, st, src, dst, lane0, total, sio, dio); break;
-        case 5: fused_pass<5, INV, STORE, LIN>(d, st, src, dst, lane0, total, sio, dio); break;
-        case 7: fused_pass<7, INV, STORE, LIN>(d, st, src, dst, lane0, total, sio, dio); break;
-        case 6: fused_pass<6, INV, STORE, LIN>(d, st, src, dst, lane0, total, sio, dio); break;
-        case 8: fused_pass<8, INV, STORE, LIN>(d, st, src, dst, lane0, total, sio, dio); break;
-        case 9: fused_pass<9, INV, STORE, LIN>(d, st, src, dst, lane0, total, sio, dio); break;
-        case 10: fused_pass<10, INV, STORE, LIN>(d, st, src, dst, lane0, total, sio, dio); break;
-        case 11: fused_pass<11, INV, STORE, LIN>(d, st, src, dst, lane0, total, sio, dio); break;
-        case 12: fused_pass<12, INV, STORE, LIN>(d, st, src, dst, lane0, total, sio, dio); break;
-        case 13: fused_pass<13, INV, STORE, LIN>(d, st, src, dst, lane0, total, sio, dio); break;
-        case 14: fused_pass<14, INV, STORE, LIN>(d, st, src, dst, lane0, total, sio, dio); break;
-        case 15: fused_pass<15, INV, STORE, LIN>(d, st, src, dst, lane0, total, sio, dio); break;
-        case 16: fused_pass<16, INV, STORE, LIN>(d, st, src, dst, lane0, total, sio, dio); break;
+        case 2: fused_pass<2, INV, STORE, LIN>(d, st, src, dst, lane0, total, sio, dio, only); break;
+        case 3: fused_pass<3, INV, STORE, LIN>(d, st, src, dst, lane0, total, sio, dio, only); break;
+        case 4: fused_pass<4, INV, STORE, LIN>(d, st, src, dst, lane0, total, sio, dio, only); break;
+        case 5: fused_pass<5, INV, STORE, LIN>(d, st, src, dst, lane0, total, sio, dio, only); break;
+        case 7: fused_pass<7, INV, STORE, LIN>(d, st, src, dst, lane0, total, sio, dio, only); break;
+        case 6: fused_pass<6, INV, STORE, LIN>(d, st, src, dst, lane0, total, sio, dio, only); break;
+        case 8: fused_pass<8, INV, STORE, LIN>(d, st, src, dst, lane0, total, sio, dio, only); break;
+        case 9: fused_pass<9, INV, STORE, LIN>(d, st, src, dst, lane0, total, sio, dio, only); break;
+        case 10: fused_pass<10, INV, STORE, LIN>(d, st, src, dst, lane0, total, sio, dio, only); break;
+        case 11: fused_pass<11, INV, STORE, LIN>(d, st, src, dst, lane0, total, sio, dio, only); break;
+        case 12: fused_pass<12, INV, STORE, LIN>(d, st, src, dst, lane0, total, sio, dio, only); break;
+        case 13: fused_pass<13, INV, STORE, LIN>(d, st, src, dst, lane0, total, sio, dio, only); break;
+        case 14: fused_pass<14, INV, STORE, LIN>(d, st, src, dst, lane0, total, sio, dio, only); break;
+        case 15: fused_pass<15, INV, STORE, LIN>(d, st, src, dst, lane0, total, sio, dio, only); break;
+        case 16: fused_pass<16, INV, STORE, LIN>(d, st, src, dst, lane0, total, sio, dio, only); break;
         default: break;
     }
 }
@@ -1680,7 +1689,7 @@ __device__ __forceinline__ void fused_dispatch(int P, const PassDesc& d, const I
 // (its planner clears d.tc) to keep its instruction footprint small.
 template <bool INV, bool SPEC = true, bool TC = true, int STORE = STORE_ANY>
 __device__ __forceinline__ void tile_body_reg(const PassDesc& d, const PassExtra& x, uint32_t tile,
-                                              vec2_t* sm) {
+                                              vec2_t* sm, const uint32_t* only = nullptr) {
     const uint32_t total = d.batch * d.lanes_j;
     const uint32_t lane0 = tile * d.C;
     const int np = d.nrad;
@@ -1741,7 +1750,7 @@ __device__ __forceinline__ void tile_body_reg(const PassDesc& d, const PassExtra
             tc_pass16<INV>(d, x.step[p], src, dst, lane0, total, sio, dio, Fr, Fi, Gm);
         else
 #endif
-            fused_dispatch<INV, STORE, kLin>(d.rad[p], d, x.step[p], src, dst, lane0, total, sio, dio);
+            fused_dispatch<INV, STORE, kLin>(d.rad[p], d, x.step[p], src, dst, lane0, total, sio, dio, only);
         // (also after the last stage: a barrier that depends on `last` makes the
         // compiler spill the values of every radix around it; with the
         // tensor-core stage it is the other way round)

@@ -112,8 +112,9 @@ __device__ __forceinline__ void fx_spec_exchange(const PassDesc& d, cfx_t* buf, 
     }
 }
 
-// The stage after stages multiplying to NS > 1, and those after it.
-template <uint32_t R, uint32_t NS, int IDX>
+// The stage after stages multiplying to NS > 1, and those after it.  OTHERS: the
+// lanes left to the FP64 body are not stored.
+template <uint32_t R, uint32_t NS, int IDX, bool OTHERS>
 __device__ __forceinline__ void fx_spec_later(const PassDesc& d, cfx_t* buf, uint32_t* words,
                                               uint32_t lane0, uint32_t total) {
     constexpr int P = fx_spec_radix(R, NS);
@@ -163,6 +164,7 @@ __device__ __forceinline__ void fx_spec_later(const PassDesc& d, cfx_t* buf, uin
 #pragma unroll
         for (int g = 0; g < G; ++g) {
             const uint32_t it = threadIdx.x + g * blockDim.x;
+            if (OTHERS && words[(kFxRows + 1) * d.C + c[g]]) continue;
             if (it < items && lane0 + c[g] < total) {
                 constexpr int P0 = fx_spec_radix(R, 1);
                 const int eb = fx_first_exp(words[c[g]], P0, pre) +
@@ -173,21 +175,23 @@ __device__ __forceinline__ void fx_spec_later(const PassDesc& d, cfx_t* buf, uin
     } else {
         __syncthreads();
         fx_spec_exchange<P, G, R, NS>(d, buf, words + (IDX + 1) * d.C, c, jj, v, false);
-        fx_spec_later<R, NS * P, IDX + 1>(d, buf, words, lane0, total);
+        fx_spec_later<R, NS * P, IDX + 1, OTHERS>(d, buf, words, lane0, total);
     }
 }
 
 // The closer look at a tile of lanes of R points (a power of two) with one that
-// may need the FP64 body (fx_beyond, fx_apart): true if one does.  In fp64_tile.cu,
-// out of the way of the other tiles' code (65536 x 64 points 48.1 us with it in
-// line, 46.4 so; 320 x 8192 96.8 and 93.0).
-__device__ bool fx_spec_apart(const PassDesc& d, uint32_t R, uint32_t* words, uint32_t lane0, uint32_t total,
-                              int span);
+// may need the FP64 body (fx_beyond, fx_apart).  In fp64_tile.cu, out of the way
+// of the other tiles' code (65536 x 64 points 48.1 us with it in line, 46.4 so;
+// 320 x 8192 96.8 and 93.0).
+__device__ FxLeft fx_spec_look(const PassDesc& d, uint32_t R, uint32_t* words, uint32_t lane0, uint32_t total,
+                               int span);
 
-// One tile (C * R <= 8 points a thread); false (with nothing written) when it
-// is one for the FP64 body.
-template <uint32_t R>
-__device__ __forceinline__ bool fx_spec_tile(const PassDesc& d, uint32_t tile, unsigned char* smem) {
+// One tile (C * R <= 8 points a thread), and what of it is left for the FP64
+// body: with anything left nothing is written, and the tile runs again as OTHERS
+// (fx_left_row is set), which writes the other lanes.  (The fast form would pay
+// for skipping lanes: 4096^2 both ways 1357 us, 1398 with the test at its stores.)
+template <uint32_t R, bool OTHERS = false>
+__device__ __forceinline__ FxLeft fx_spec_tile(const PassDesc& d, uint32_t tile, unsigned char* smem) {
     constexpr int P = fx_spec_radix(R, 1);
     constexpr int G = 8 / P;
     constexpr uint32_t M = R / P;
@@ -197,7 +201,7 @@ __device__ __forceinline__ bool fx_spec_tile(const PassDesc& d, uint32_t tile, u
     cfx_t* buf = reinterpret_cast<cfx_t*>(smem);
     uint32_t* words = reinterpret_cast<uint32_t*>(smem + d.fx_words);
     uint32_t* both = words + kFxRows * d.C;  // (fx_guard_row: at most four stages)
-    for (uint32_t i = threadIdx.x; i < (kFxRows + fx_guard_rows(R)) * d.C; i += blockDim.x) words[i] = 0;
+    for (uint32_t i = threadIdx.x; i < (kFxRows + (OTHERS ? 1 : fx_guard_rows(R))) * d.C; i += blockDim.x) words[i] = 0;
     const bool lane_mode = d.load_mode == MODE_LANE;
     uint32_t c[G], jj[G];
     double2 raw[G][P];
@@ -272,7 +276,7 @@ __device__ __forceinline__ bool fx_spec_tile(const PassDesc& d, uint32_t tile, u
 #pragma unroll
     for (int g = 0; g < G; ++g) {
         // (a chirp turns every element, so nothing stays apart)
-        {
+        if constexpr (!OTHERS) {
             const uint32_t most = words[c[g]], near = fx_near(most, fx_span(P));
             bool look = !chirp && most != 0 && both[c[g]] < near;
             if (!lane_mode && __any_sync(0xffffffffu, look)) {
@@ -321,10 +325,12 @@ __device__ __forceinline__ bool fx_spec_tile(const PassDesc& d, uint32_t tile, u
         }
     }
     fx_spec_exchange<P, G, R, 1>(d, buf, words + d.C, c, jj, v, lane_mode);
-    if (__builtin_expect(__syncthreads_or(rare), 0) && fx_spec_apart(d, R, words, lane0, total, fx_span(P)))
-        return false;
-    fx_spec_later<R, P, 1>(d, buf, words, lane0, total);
-    return true;
+    if (__builtin_expect(__syncthreads_or(rare), 0)) {
+        const FxLeft left = fx_spec_look(d, R, words, lane0, total, fx_span(P));
+        if (left != FX_NOTHING) return left;
+    }
+    fx_spec_later<R, P, 1, OTHERS>(d, buf, words, lane0, total);
+    return FX_NOTHING;
 }
 
 }  // namespace kfft

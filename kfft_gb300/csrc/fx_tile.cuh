@@ -24,11 +24,13 @@
 // 16384 x 1000 417 against 566.  The FP64 body these tiles replace ran the
 // uneven batch of 256 in 1672 us, they run it in 862.
 //
-// A tile that holds an infinity, a NaN, a magnitude from 2^768 on or a lane
-// whose largest is below 2^-767 is left to the FP64 body, which treats them as
-// IEEE arithmetic does (smaller values beside larger ones shift out), and so is
-// one with a lane whose small parts doubles would keep apart from its large
-// ones (fx_apart in fx_math.cuh).  Telling the lanes costs up to 6% (65536 x 64
+// A lane that holds an infinity, a NaN, a magnitude from 2^768 on or nothing
+// from 2^-767 on is left to the FP64 body, which treats them as IEEE arithmetic
+// does (smaller values beside larger ones shift out), and so is one whose small
+// parts doubles would keep apart from its large ones (fx_apart in fx_math.cuh):
+// the lane, not its tile, so that what becomes of a sequence does not depend on
+// those beside it.
+// Telling the lanes costs up to 6% (65536 x 64
 // points 43.8 -> 46.4 us, 4096 x 1000 116 -> 119, uneven batch of 256 829 -> 862,
 // 4096^2 both ways level); real values in the complex form, 4096 x 1000 points,
 // take the closer look and 136; a tile that leaves after it has spent 10 to 15% of
@@ -48,6 +50,10 @@ constexpr uint32_t kFxExpLow = 256, kFxExpHigh = 1791;
 __device__ __forceinline__ bool fx_beyond(uint32_t most) {
     return most != 0 && ((most >> 20) < kFxExpLow || (most >> 20) >= kFxExpHigh);
 }
+
+// What a fixed-point tile leaves to the FP64 body: nothing, the lanes named in
+// fx_left_row, or all (nothing written).
+enum FxLeft : uint32_t { FX_NOTHING = 0, FX_SOME = 1, FX_ALL = 2 };
 
 __device__ __forceinline__ FxTw fx_tw_load(const FxTw* p) {
     const int4 v = __ldg(reinterpret_cast<const int4*>(p));
@@ -108,6 +114,29 @@ __device__ __forceinline__ uint32_t fx_holds(double2 x, uint32_t near) {
 // elements' smaller parts (a lane where it is near the largest stays without a
 // closer look), and what the lane holds (FX_HAS_RE ...)
 __device__ __forceinline__ uint32_t fx_guard_row(const PassDesc& d) { return max(uint32_t(d.nrad), kFxRows); }
+
+// the second of them, in the end: not zero for the lanes that FP64 has to do
+__device__ __forceinline__ uint32_t* fx_left_row(const PassDesc& d, unsigned char* smem) {
+    return reinterpret_cast<uint32_t*>(smem + d.fx_words) + (fx_guard_row(d) + 1) * d.C;
+}
+
+// Turns what the lanes hold into that; every thread gets the outcome.  pair(c):
+// lane c has a pair that `holds` does not say.
+template <class Pair>
+__device__ __forceinline__ FxLeft fx_settle(const PassDesc& d, const uint32_t* words, uint32_t* holds,
+                                            uint32_t lane0, uint32_t total, Pair pair) {
+    bool some = false, all = true;
+    for (uint32_t c = threadIdx.x; c < d.C; c += blockDim.x) {
+        uint32_t f = holds[c];
+        if (fx_apart(f) && pair(c)) f |= FX_PAIR;
+        const bool left = fx_beyond(words[c]) || fx_apart(f);
+        holds[c] = left;
+        some = some || left;
+        all = all && (left || lane0 + c >= total);
+    }
+    if (!__syncthreads_or(some)) return FX_NOTHING;
+    return __syncthreads_and(all) ? FX_ALL : FX_SOME;
+}
 
 // sequence and lane index of lane g of a pass
 __device__ __forceinline__ void fx_lane(const PassDesc& d, uint32_t g, uint32_t& b, uint32_t& j) {
@@ -176,10 +205,10 @@ struct FxWalk {
 };
 
 // Reads the tile and leaves it in `buf` as integers (prologue and outer
-// twiddle applied); false when the tile is one for the FP64 body.  words[c]
-// becomes the largest magnitude word of lane c.
-__device__ __forceinline__ bool fx_read(const PassDesc& d, cfx_t* buf, uint32_t* words,
-                                        const FxLane* lanes) {
+// twiddle applied), unless all of it is for the FP64 body.  words[c] becomes the
+// largest magnitude word of lane c.
+__device__ __forceinline__ FxLeft fx_read(const PassDesc& d, cfx_t* buf, uint32_t* words,
+                                          const FxLane* lanes, uint32_t lane0, uint32_t total) {
     const uint32_t elems = d.C * d.R;
     const bool lane_mode = d.load_mode == MODE_LANE;
     const uint64_t step = uint64_t(d.lanes_j) * d.in_es;
@@ -245,28 +274,27 @@ __device__ __forceinline__ bool fx_read(const PassDesc& d, cfx_t* buf, uint32_t*
     // (a chirp turns every element, so nothing stays apart)
     const bool chirped = d.pro_op == PRO_CHIRP;
     const int span = fx_span(d.rad[0]);
-    bool rare = false, beyond = false;
-    for (uint32_t c = threadIdx.x; c < d.C; c += blockDim.x) {
-        beyond = beyond || fx_beyond(words[c]);
-        rare = rare || (!chirped && words[c] != 0 && both[c] < fx_near(words[c], span));
-    }
-    if (__syncthreads_or(rare || beyond)) {
-        if (__syncthreads_or(beyond)) return false;
+    FxLeft left = FX_NOTHING;
+    bool rare = false;
+    for (uint32_t c = threadIdx.x; c < d.C; c += blockDim.x)
+        rare = rare || fx_beyond(words[c]) || (!chirped && words[c] != 0 && both[c] < fx_near(words[c], span));
+    if (__syncthreads_or(rare)) {
         uint32_t* holds = both + d.C;
-        FxWalk w(d, false);
+        if (!chirped) {
+            FxWalk w(d, false);
 #pragma unroll 1
-        for (uint32_t i = threadIdx.x; i < elems; i += blockDim.x, w.next(d)) {
-            const double2* lane = reinterpret_cast<const double2*>(&buf[w.c * d.lane_stride]);
-            const uint32_t near = fx_near(words[w.c], span), r1 = w.r + 1 == d.R ? 0 : w.r + 1;
-            const double2 x = lane[pad(w.r)], y = lane[pad(r1)];
-            uint32_t f = fx_holds(x, near);
-            if (max(fx_mag(x.x), fx_mag(x.y)) >= near && max(fx_mag(y.x), fx_mag(y.y)) >= near) f |= FX_PAIR;
-            if (f) atomicOr(&holds[w.c], f);
+            for (uint32_t i = threadIdx.x; i < elems; i += blockDim.x, w.next(d)) {
+                const double2* lane = reinterpret_cast<const double2*>(&buf[w.c * d.lane_stride]);
+                const uint32_t near = fx_near(words[w.c], span), r1 = w.r + 1 == d.R ? 0 : w.r + 1;
+                const double2 x = lane[pad(w.r)], y = lane[pad(r1)];
+                uint32_t f = fx_holds(x, near);
+                if (max(fx_mag(x.x), fx_mag(x.y)) >= near && max(fx_mag(y.x), fx_mag(y.y)) >= near) f |= FX_PAIR;
+                if (f) atomicOr(&holds[w.c], f);
+            }
+            __syncthreads();
         }
-        __syncthreads();
-        bool apart = false;
-        for (uint32_t c = threadIdx.x; c < d.C; c += blockDim.x) apart = apart || fx_apart(holds[c]);
-        if (__syncthreads_or(apart)) return false;
+        left = fx_settle(d, words, holds, lane0, total, [](uint32_t) { return false; });
+        if (left == FX_ALL) return left;
     }
     // each thread its own elements again: integers against their lane's scale
     const bool outer = d.Ns > 1, chirp = chirped, inv = d.inv != 0;
@@ -289,7 +317,7 @@ __device__ __forceinline__ bool fx_read(const PassDesc& d, cfx_t* buf, uint32_t*
         *p = v;
         w.next(d);
     }
-    return true;
+    return left;
 }
 
 // One stage of radix P, shared memory to shared memory (one buffer where
@@ -373,9 +401,9 @@ __device__ __forceinline__ void fx_exponents(const PassDesc& d, uint32_t* words)
     }
 }
 
-// Writes the tile through the epilogue.
+// Writes the tile (but for the lanes in `skip`, if given) through the epilogue.
 __device__ __forceinline__ void fx_write(const PassDesc& d, const cfx_t* buf, const uint32_t* words,
-                                         const FxLane* lanes) {
+                                         const FxLane* lanes, const uint32_t* skip) {
     const uint32_t elems = d.C * d.R;
     const bool inv = d.inv != 0;
     const uint32_t op = d.epi_op;
@@ -390,7 +418,7 @@ __device__ __forceinline__ void fx_write(const PassDesc& d, const cfx_t* buf, co
 #pragma unroll 2
     for (uint32_t i = threadIdx.x; i < elems; i += blockDim.x, w.next(d)) {
         const FxLane& l = lanes[w.c];
-        if (l.b == kFxDead) continue;
+        if (l.b == kFxDead || (skip && skip[w.c])) continue;
         const uint32_t k = l.k + w.r * d.Ns;
         if (op == EPI_CHIRP && k >= d.epi_bound) continue;
         cfx_t u = buf[w.c * d.lane_stride + pad(w.r)];
@@ -426,20 +454,21 @@ __device__ __forceinline__ void fx_write(const PassDesc& d, const cfx_t* buf, co
     }
 }
 
-// One tile of a pass in fixed point; false (with nothing written) when the
-// tile is one for the FP64 body.  Shared memory: the exchange buffers (one
-// where d.inplace), at byte d.fx_words a row of words per stage, and after
-// them the lane table.
-__device__ __forceinline__ bool fx_tile(const PassDesc& d, const PassExtra& x, uint32_t tile,
-                                        unsigned char* smem) {
+// One tile of a pass in fixed point, and what of it is left for the FP64 body.
+// Shared memory: the exchange buffers (one where d.inplace), at byte d.fx_words
+// a row of words per stage and the guard's, and after them the lane table.
+__device__ __forceinline__ FxLeft fx_tile(const PassDesc& d, const PassExtra& x, uint32_t tile,
+                                          unsigned char* smem) {
     cfx_t* bufA = reinterpret_cast<cfx_t*>(smem);
     cfx_t* bufB = d.inplace ? bufA : bufA + d.C * d.lane_stride + 1;
     uint32_t* words = reinterpret_cast<uint32_t*>(smem + d.fx_words);
     FxLane* lanes = reinterpret_cast<FxLane*>(smem + d.fx_lanes);
     for (uint32_t i = threadIdx.x; i < (fx_guard_row(d) + 2) * d.C; i += blockDim.x) words[i] = 0;
-    fx_lanes(d, lanes, tile * d.C, d.batch * d.lanes_j);
+    const uint32_t lane0 = tile * d.C, total = d.batch * d.lanes_j;
+    fx_lanes(d, lanes, lane0, total);
     __syncthreads();
-    if (!fx_read(d, bufA, words, lanes)) return false;
+    const FxLeft left = fx_read(d, bufA, words, lanes, lane0, total);
+    if (left == FX_ALL) return left;
     __syncthreads();
     cfx_t* src = bufA;
 #pragma unroll 1
@@ -458,18 +487,21 @@ __device__ __forceinline__ bool fx_tile(const PassDesc& d, const PassExtra& x, u
         __syncthreads();
         src = dst;
     }
-    fx_write(d, src, words, lanes);
-    return true;
+    fx_write(d, src, words, lanes, left == FX_SOME ? fx_left_row(d, smem) : nullptr);
+    return left;
 }
 
-// the FP64 body (fp64_tile.cu): only tiles the fixed-point ones turn down run it
-__device__ void fp64_tile(const PassDesc& d, const PassExtra& x, uint32_t tile, unsigned char* smem);
+// The FP64 body (fp64_tile.cu) for what a fixed-point tile leaves.  (A
+// compile-time tile stops before it stores anything; its other lanes run again
+// first.)
+__device__ void fp64_tile(const PassDesc& d, const PassExtra& x, uint32_t tile, unsigned char* smem,
+                          FxLeft left);
 
 // a register tile of the double build
 __device__ __forceinline__ void double_tile(const PassDesc& d, const PassExtra& x, uint32_t tile,
                                             unsigned char* smem) {
-    if (d.fx && fx_tile(d, x, tile, smem)) return;
-    fp64_tile(d, x, tile, smem);
+    const FxLeft left = d.fx ? fx_tile(d, x, tile, smem) : FX_ALL;
+    if (left != FX_NOTHING) fp64_tile(d, x, tile, smem, left);
 }
 
 }  // namespace kfft

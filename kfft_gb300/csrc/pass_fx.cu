@@ -23,7 +23,8 @@ template <uint32_t R>
 __global__ void __launch_bounds__(kFxSpecThreads, 2) k_fx_spec(const __grid_constant__ PassDesc d,
                                                                const __grid_constant__ PassExtra x) {
     extern __shared__ __align__(16) unsigned char smem_raw[];
-    if (!fx_spec_tile<R>(d, blockIdx.x, smem_raw)) fp64_tile(d, x, blockIdx.x, smem_raw);
+    const FxLeft left = fx_spec_tile<R>(d, blockIdx.x, smem_raw);
+    if (left != FX_NOTHING) fp64_tile(d, x, blockIdx.x, smem_raw, left);
 }
 
 #if KFFT_FX_PART == 0

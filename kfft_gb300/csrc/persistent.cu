@@ -67,21 +67,21 @@ __device__ __forceinline__ void run_item(const PassDesc& d, const PassExtra& x, 
                                          vec2_t* buf) {
 #if !defined(KFFT_HALF_SCALAR)
     unsigned char* smem = reinterpret_cast<unsigned char*>(buf);
-    bool ok = false;
+    FxLeft left = FX_ALL;
     if (d.fx) {
         switch (d.spec) {
-            case 4: ok = fx_spec_tile<16>(d, tile, smem); break;
-            case 5: ok = fx_spec_tile<32>(d, tile, smem); break;
-            case 6: ok = fx_spec_tile<64>(d, tile, smem); break;
-            case 7: ok = fx_spec_tile<128>(d, tile, smem); break;
-            case 8: ok = fx_spec_tile<256>(d, tile, smem); break;
-            case 9: ok = fx_spec_tile<512>(d, tile, smem); break;
-            case 10: ok = fx_spec_tile<1024>(d, tile, smem); break;
-            case 11: ok = fx_spec_tile<2048>(d, tile, smem); break;
-            default: ok = fx_tile(d, x, tile, smem); break;
+            case 4: left = fx_spec_tile<16>(d, tile, smem); break;
+            case 5: left = fx_spec_tile<32>(d, tile, smem); break;
+            case 6: left = fx_spec_tile<64>(d, tile, smem); break;
+            case 7: left = fx_spec_tile<128>(d, tile, smem); break;
+            case 8: left = fx_spec_tile<256>(d, tile, smem); break;
+            case 9: left = fx_spec_tile<512>(d, tile, smem); break;
+            case 10: left = fx_spec_tile<1024>(d, tile, smem); break;
+            case 11: left = fx_spec_tile<2048>(d, tile, smem); break;
+            default: left = fx_tile(d, x, tile, smem); break;
         }
     }
-    if (!ok) fp64_tile(d, x, tile, smem);
+    if (left != FX_NOTHING) fp64_tile(d, x, tile, smem, left);
 #else
     if (d.inv) tile_body_reg<true, true, false>(d, x, tile, buf);
     else tile_body_reg<false, true, false>(d, x, tile, buf);
