@@ -287,11 +287,13 @@ void launch_pass_reg(const PassDesc& d, const PassExtra& x, cudaStream_t st) {
             const int per_sm = f ? prepare((const void*)f, smem) : -1;
             const uint32_t grid = uint32_t(std::max(per_sm, 0)) * uint32_t(sm_count());
             uint32_t* fail = wait_flags();
-            // from where k_pass_pipe's two CTAs an SM start a third round (608
-            // tiles; us there and here: 16 points 700 tiles 20.6, 18.0, 760 tiles
-            // 24.7, 20.6, 911 tiles 24.7, 20.6; 256 points 760 tiles 12.4, 10.4;
-            // 4096 points level; at 608 tiles 12.4, 14.4)
-            if (fail && per_sm > 0 && 3 * d.tiles > 4 * grid) {
+            // from two full rounds on, 912 tiles.  (From where k_pass_pipe's two CTAs
+            // an SM start a third round, 609 tiles, this kernel itself is no slower, us
+            // there and here: 16 points 760 tiles 24.7, 20.6, 256 points 12.4, 10.4,
+            // 4096 points level; but a synchronous call that has launched it asks for
+            // failed waits behind it: the real 2D forward and inverse of 877 x 2500, whose
+            // inverse has 626 tiles, 248 us with k_pass_pipe there, 265 with this.)
+            if (fail && per_sm > 0 && d.tiles >= 2 * grid) {
                 f<<<grid, kPassThreads, smem, st>>>(d, fail + wait_slot(), bulk_wait_polls());
                 note_cuda_error(cudaGetLastError());
                 note_bulk_launch();
