@@ -84,3 +84,39 @@ def test_queue(lib):
     for i in range(len(lengths)):
         if i not in (1, 4):
             assert np.array_equal(got[i], ref[i]), i
+
+
+@pytest.mark.parametrize("n", [8, 45, 64, 512, 1000, 2048, 8192, 257])
+def test_in_place(lib, n):
+    """The tiles that do some lanes after the others, on one buffer."""
+    torch = pytest.importorskip("torch")
+    mixed = noise((11, n), 3 * n)
+    mixed[[1, 2, 4, 5, 6, 8, 9, 10]] = odd_ones(n)
+    x = torch.from_numpy(mixed).cuda()
+    y = torch.empty_like(x)
+    for flags in (K.FLAG_NORMAL, K.FLAG_INVERSE):
+        z = x.clone()
+        p = lib._plan("kfft_config_cpx", n, flags)
+        assert lib.L.kfft_eval_cpx_batch(p, x.data_ptr(), y.data_ptr(), 11) == 0
+        assert lib.L.kfft_eval_cpx_batch(p, z.data_ptr(), z.data_ptr(), 11) == 0
+        lib.cleanup(p)
+        assert np.array_equal(y.cpu().numpy(), z.cpu().numpy(), equal_nan=True)
+
+
+@pytest.mark.parametrize("y,x", [(64, 40), (512, 36), (45, 40), (4096, 20), (8192, 20)])
+def test_columns_in_place(lib, y, x):
+    """Likewise down columns, of which every fifth row-transforms to nearly real
+    values."""
+    torch = pytest.importorskip("torch")
+    a = noise((y, x), x)
+    cols = np.fft.fft(a, axis=1)
+    cols[:, ::5].imag *= 2.0 ** -20
+    t = torch.from_numpy(np.ascontiguousarray(np.fft.ifft(cols, axis=1))).cuda()
+    out, z = torch.empty_like(t), t.clone()
+    p = lib._plan("kfft_config2_cpx", x, y, K.FLAG_NORMAL)
+    assert lib.L.kfft_eval2_cpx(p, t.data_ptr(), out.data_ptr()) == 0
+    assert lib.L.kfft_eval2_cpx(p, z.data_ptr(), z.data_ptr()) == 0
+    lib.cleanup(p)
+    assert torch.equal(out, z)
+    ref = torch.fft.fft2(t)
+    assert float(torch.linalg.norm(out - ref) / torch.linalg.norm(ref)) <= 1e-15
