@@ -30,12 +30,12 @@
 // parts doubles would keep apart from its large ones (fx_apart in fx_math.cuh):
 // the lane, not its tile, so that what becomes of a sequence does not depend on
 // those beside it.
-// Telling the lanes costs up to 6% (65536 x 64
-// points 43.8 -> 46.4 us, 4096 x 1000 116 -> 119, uneven batch of 256 829 -> 862,
-// 4096^2 both ways level); real values in the complex form, 4096 x 1000 points,
-// take the closer look and 136; a tile that leaves after it has spent 10 to 15% of
-// its FP64 time (256 x 4096 nearly real points 121 us, in FP64 from the start
-// 106).
+//
+// Telling the lanes costs up to 6% (65536 x 64 points 43.8 -> 46.4 us, 4096 x 1000
+// 116 -> 119, uneven batch of 256 829 -> 862, 4096^2 both ways level); real values
+// in the complex form, 4096 x 1000 points, take the closer look and 136; a tile
+// that leaves after it has spent 10 to 15% of its FP64 time (256 x 4096 nearly
+// real points 121 us, in FP64 from the start 106).
 #pragma once
 
 #include "fft_device.cuh"
